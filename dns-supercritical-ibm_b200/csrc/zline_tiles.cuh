@@ -27,6 +27,7 @@
 #include "cp_async.cuh"
 #include "div_rn.cuh"
 #include "fft_pass.cuh"
+#include "thomas_block.cuh"
 #include "tma_util.cuh"
 
 struct prj_plan;
@@ -81,7 +82,8 @@ PRJ_PASS_PLANS(PRJ_ZL_LAYOUT_CHECK)
 #undef PRJ_ZL_LAYOUT_CHECK
 
 // Shared memory of a tile: 128 bytes of alignment slack, NS mbarriers (128 bytes),
-// NS row stages of zl_slot_bytes each (128-byte aligned), then the pivot ring.  A stage
+// NS row stages of zl_slot_bytes each (128-byte aligned), then the pivot ring and the
+// planes' a and a00.  A stage
 // holds yb rows in the padded layout of the FFT passes: each group of 8 complex values is
 // followed by one pad slot, which is what a tensor-map box of 9 complex values per group
 // (the 9th out of bounds, zero-filled) writes.
@@ -92,9 +94,9 @@ __host__ __device__ inline size_t zl_slot_bytes(int n, int yb) { return ((size_t
 // (zline_smem bytes).  Each stage's rows arrive by one tensor-map copy (`tmap`:
 // zline_tmap's 4-D view of the spectrum) issued by thread 0 and completed on an mbarrier;
 // the pivot rows are cp.async copies (their pieces are permuted).  Every mbarrier wait is
-// bounded: on a timeout the tile raises *a.err, waits (bounded) for its copies in flight
+// bounded; UP planes of the forward sweep are unrolled: on a timeout the tile raises *a.err, waits (bounded) for its copies in flight
 // and returns.
-template <class PL, int NS, int LPT, int NT>
+template <class PL, int NS, int LPT, int NT, int UP = 2>
 __device__ __forceinline__ void zline_tile(const ZLineArgs& a, const void* tmap, int kx, unsigned char* zsm) {
     constexpr int n = PL::n;
     static_assert(NT * LPT >= n, "every line has a thread");
@@ -106,6 +108,7 @@ __device__ __forceinline__ void zline_tile(const ZLineArgs& a, const void* tmap,
     const size_t slot_bytes = zl_slot_bytes(n, yb);
     unsigned char* rslots = base + 128;
     double* dring = reinterpret_cast<double*>(rslots + NS * slot_bytes);
+    double* aring = dring + (size_t)NS * yb * mzs;  // a and a00 of each stage's planes
     auto stage = [&](int s) { return reinterpret_cast<double2*>(rslots + s * slot_bytes); };
     if (tid == 0) {
 #pragma unroll
@@ -117,18 +120,17 @@ __device__ __forceinline__ void zline_tile(const ZLineArgs& a, const void* tmap,
     uint32_t pending = 0;  // bit s: stage s has a copy in flight (the same in every thread)
 
     // this thread's lines
-    int slot[LPT], kzs[LPT];
+    int slot[LPT], at[LPT], kzs[LPT];
     bool is00[LPT];
 #pragma unroll
     for (int q = 0; q < LPT; q++) {
         slot[q] = tid + q * NT;
-        const int kz = slot[q] < n ? a.kz_of_slot[slot[q]] : 0;
+        at[q] = slot[q] < n ? slot[q] : 0;
+        const int kz = a.kz_of_slot[at[q]];
         const int kf = kz <= n - kz ? kz : n - kz;
         kzs[q] = 2 * zl_piece(kf >> 1) + (kf & 1);  // position in a shared pivot row
         is00[q] = (kx == 0 && kz == 0);
     }
-    const double* bA = a.bands;
-    const double* bA0 = a.bands + 3 * ny;
 
     // chunk c (planes c yb ..) into stage s with the rows of table tab (pivots on the way
     // up, back-substitution factors on the way down): the rows by one tensor-map copy (a
@@ -148,6 +150,10 @@ __device__ __forceinline__ void zline_tile(const ZLineArgs& a, const void* tmap,
             for (int i = tid; i < nr * hp; i += NT) {
                 const int r = i / hp, j = i - r * hp;
                 cp_async(dbuf + (size_t)r * mzs + 2 * zl_piece(j), tab + ((size_t)(y0 + r) * nh + kx) * mzp + 2 * j, 16);
+            }
+            for (int i = tid; tab == a.piv && i < 2 * nr; i += NT) {
+                const int k = i < nr ? 0 : 3, r = i < nr ? i : i - nr;
+                cp_async(aring + (size_t)(2 * s + (k ? 1 : 0)) * yb + r, a.bands + (size_t)k * ny + y0 + r, 8);
             }
         }
         cp_async_commit();
@@ -191,26 +197,42 @@ __device__ __forceinline__ void zline_tile(const ZLineArgs& a, const void* tmap,
         }
         double2* buf = stage(s);
         const double* dbuf = dring + (size_t)s * yb * mzs;
+        const double* abuf = aring + (size_t)2 * s * yb;
         dif_passes_shared<-1, PL, 0, PL::P>(buf, nr, n, a.tw);  // barrier after every pass
+        // plane by plane (lines past n run along on line 0's values and store nothing); a
+        // quotient that may differ is noticed at the end of the chunk, whose inputs the stage
+        // still holds
+        double2 below[LPT];
+#pragma unroll
+        for (int q = 0; q < LPT; q++) below[q] = prev[q];
+        unsigned outside = 0;
+#pragma unroll UP
         for (int r = 0; r < nr; r++) {
-            const int y = y0 + r;
-            double2* grow = a.X + ((size_t)y * nh + kx) * n;
+            double2 v[LPT][1];
+            double D[LPT][1], rD[LPT][1], av[LPT][1];
 #pragma unroll
             for (int q = 0; q < LPT; q++) {
-                if (slot[q] < n) {
-                    double2 v = buf[sidx<true>(r * n + slot[q])];
-                    const double D = dbuf[(size_t)r * mzs + kzs[q]];
-                    const double rD = __drcp_rn(D);  // off the recurrence's chain
-                    if (y == 0) {
-                        v.x = div_by_recip(v.x, D, rD);
-                        v.y = div_by_recip(v.y, D, rD);
-                    } else {
-                        const double av = is00[q] ? bA0[y] : bA[y];
-                        v.x = div_by_recip(__dsub_rn(v.x, __dmul_rn(av, prev[q].x)), D, rD);
-                        v.y = div_by_recip(__dsub_rn(v.y, __dmul_rn(av, prev[q].y)), D, rD);
-                    }
-                    prev[q] = v;
-                    grow[slot[q]] = v;
+                v[q][0] = buf[sidx<true>(r * n + at[q])];
+                D[q][0] = dbuf[(size_t)r * mzs + kzs[q]];
+                rD[q][0] = __drcp_rn(D[q][0]);  // off the recurrence's chain
+                av[q][0] = y0 + r > 0 ? abuf[(is00[q] ? yb : 0) + r] : 0.0;
+            }
+            sweep_up<1, LPT>(v, D, rD, av, 1, prev, outside);
+            double2* grow = a.X + ((size_t)(y0 + r) * nh + kx) * n;
+#pragma unroll
+            for (int q = 0; q < LPT; q++)
+                if (slot[q] < n) grow[slot[q]] = v[q][0];
+        }
+        if (outside) {
+#pragma unroll
+            for (int q = 0; q < LPT; q++) prev[q] = below[q];
+            for (int r = 0; r < nr; r++) {
+                double2* grow = a.X + ((size_t)(y0 + r) * nh + kx) * n;
+#pragma unroll
+                for (int q = 0; q < LPT; q++) {
+                    prev[q] = step_up_safe(buf[sidx<true>(r * n + at[q])], dbuf[(size_t)r * mzs + kzs[q]],
+                                           y0 + r > 0 ? abuf[(is00[q] ? yb : 0) + r] : 0.0, prev[q]);
+                    if (slot[q] < n) grow[slot[q]] = prev[q];
                 }
             }
         }
@@ -273,9 +295,9 @@ __device__ __forceinline__ void zline_tile(const ZLineArgs& a, const void* tmap,
 // z_planes tuning or 4; prj_zline.cu)
 ZLineArgs zline_args(const prj_plan* pl);
 
-// shared memory of a tile (alignment slack, mbarriers, row stages, pivot ring)
+// shared memory of a tile (alignment slack, mbarriers, row stages, pivot ring, a and a00)
 inline size_t zline_smem(int n, int mzp, int yb, int ns) {
-    return 256 + (size_t)ns * zl_slot_bytes(n, yb) + (size_t)ns * yb * zl_mzs(mzp) * sizeof(double);
+    return 256 + (size_t)ns * zl_slot_bytes(n, yb) + (size_t)ns * yb * (zl_mzs(mzp) + 2) * sizeof(double);
 }
 
 // the 4-D tensor map of the row copies over the spectrum X (n-point z rows,

@@ -10,6 +10,7 @@
 #include "cp_async.cuh"
 #include "div_rn.cuh"
 #include "fft_pass.cuh"
+#include "thomas_block.cuh"
 
 struct prj_plan;
 
@@ -135,39 +136,37 @@ __device__ __forceinline__ void thomas_line(const ThomasArgs& a, int blk) {
     const double* dc = a.pivc + (size_t)kx * mzp + kzs;
 
     // forward sweep, y ascending
-    double2 prev = make_double2(0.0, 0.0);
+    double2 prev[1] = {make_double2(0.0, 0.0)};
     for (int y0 = 0; y0 < ny; y0 += kBlock) {
-        double2 v[kBlock];
-        double D[kBlock], av[kBlock];
+        const int nb = min(kBlock, ny - y0);
+        double2 v[1][kBlock];
+        double D[1][kBlock], rD[1][kBlock], av[1][kBlock];
 #pragma unroll
         for (int u = 0; u < kBlock; u++) {
-            const int y = y0 + u;
-            if (y < ny) {
-                v[u] = to_d2(x[(size_t)y * rstride]);
-                D[u] = d[(size_t)y * pstride];
-                av[u] = A[y];
-            }
+            const int y = min(y0 + u, ny - 1);
+            v[0][u] = to_d2(x[(size_t)y * rstride]);
+            D[0][u] = d[(size_t)y * pstride];
+            av[0][u] = y > 0 ? A[y] : 0.0;
         }
 #pragma unroll
-        for (int u = 0; u < kBlock; u++) {
-            const int y = y0 + u;
-            if (y < ny) {
-                double2 r = v[u];
-                const double rD = __drcp_rn(D[u]);  // off the recurrence's chain
-                if (y == 0) {
-                    r.x = div_by_recip(r.x, D[u], rD);
-                    r.y = div_by_recip(r.y, D[u], rD);
-                } else {
-                    r.x = div_by_recip(__dsub_rn(r.x, __dmul_rn(av[u], prev.x)), D[u], rD);
-                    r.y = div_by_recip(__dsub_rn(r.y, __dmul_rn(av[u], prev.y)), D[u], rD);
-                }
-                prev = r;
-                if (y < ny - 1) from_d2(x[(size_t)y * rstride], r);
+        for (int u = 0; u < kBlock; u++) rD[0][u] = __drcp_rn(D[0][u]);  // off the recurrence's chain
+        const double2 below = prev[0];
+        unsigned outside = 0;
+        sweep_up<kBlock, 1>(v, D, rD, av, nb, prev, outside);
+        if (!outside) {
+#pragma unroll
+            for (int u = 0; u < kBlock; u++)
+                if (y0 + u < ny - 1) from_d2(x[(size_t)(y0 + u) * rstride], v[0][u]);
+        } else {
+            prev[0] = below;
+            for (int y = y0; y < y0 + nb; y++) {
+                prev[0] = step_up_safe(to_d2(x[(size_t)y * rstride]), d[(size_t)y * pstride], y > 0 ? A[y] : 0.0, prev[0]);
+                if (y < ny - 1) from_d2(x[(size_t)y * rstride], prev[0]);
             }
         }
     }
     // backward sweep, y descending; prev holds d'_{ny-1} = x_{ny-1}
-    from_d2(x[(size_t)(ny - 1) * rstride], prev);
+    from_d2(x[(size_t)(ny - 1) * rstride], prev[0]);
     for (int y1 = ny - 2; y1 >= 0; y1 -= kBlock) {
         double2 v[kBlock];
         double cp[kBlock];
@@ -185,9 +184,9 @@ __device__ __forceinline__ void thomas_line(const ThomasArgs& a, int blk) {
             if (y >= 0) {
                 const double c = cp[u];
                 double2 r;
-                r.x = __dsub_rn(v[u].x, __dmul_rn(prev.x, c));
-                r.y = __dsub_rn(v[u].y, __dmul_rn(prev.y, c));
-                prev = r;
+                r.x = __dsub_rn(v[u].x, __dmul_rn(prev[0].x, c));
+                r.y = __dsub_rn(v[u].y, __dmul_rn(prev[0].y, c));
+                prev[0] = r;
                 from_d2(x[(size_t)y * rstride], r);
             }
         }
@@ -239,35 +238,42 @@ __device__ __forceinline__ void thomas_line_async(const ThomasArgs& a, int blk, 
     };
 #pragma unroll
     for (int b = 0; b < NS - 1; b++) issue_f(b);
-    double2 prev = make_double2(0.0, 0.0);
+    double2 prev[1] = {make_double2(0.0, 0.0)};
     for (int b = 0; b < nb; b++) {
         issue_f(b + NS - 1);
         cp_async_wait<NS - 1>();
-        const int st = b % NS;
+        const int st = b % NS, y0 = b * B, nbk = min(B, ny - y0);
+        double2 v[1][B];
+        double D[1][B], rD[1][B], av[1][B];
 #pragma unroll
         for (int u = 0; u < B; u++) {
-            const int y = b * B + u;
-            if (y < ny) {
-                double2 r = to_d2(xs(st, u));
-                const double D = ds(st, u);
-                const double rD = __drcp_rn(D);  // off the recurrence's chain
-                if (y == 0) {
-                    r.x = div_by_recip(r.x, D, rD);
-                    r.y = div_by_recip(r.y, D, rD);
-                } else {
-                    const double av = A[y];
-                    r.x = div_by_recip(__dsub_rn(r.x, __dmul_rn(av, prev.x)), D, rD);
-                    r.y = div_by_recip(__dsub_rn(r.y, __dmul_rn(av, prev.y)), D, rD);
-                }
-                prev = r;
-                if (y < ny - 1) from_d2(x[(size_t)y * rstride], r);
+            const int w = min(u, nbk - 1);
+            v[0][u] = to_d2(xs(st, w));
+            D[0][u] = ds(st, w);
+            av[0][u] = y0 + w > 0 ? A[y0 + w] : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < B; u++) rD[0][u] = __drcp_rn(D[0][u]);  // off the recurrence's chain
+        const double2 below = prev[0];
+        unsigned outside = 0;
+        sweep_up<B, 1>(v, D, rD, av, nbk, prev, outside);
+        if (!outside) {
+#pragma unroll
+            for (int u = 0; u < B; u++)
+                if (y0 + u < ny - 1) from_d2(x[(size_t)(y0 + u) * rstride], v[0][u]);
+        } else {
+            prev[0] = below;
+            for (int u = 0; u < nbk; u++) {
+                const int y = y0 + u;
+                prev[0] = step_up_safe(to_d2(xs(st, u)), ds(st, u), y > 0 ? A[y] : 0.0, prev[0]);
+                if (y < ny - 1) from_d2(x[(size_t)y * rstride], prev[0]);
             }
         }
     }
     cp_async_wait<0>();
     // the backward sweep reads what this thread just stored: complete those stores first
     __threadfence();
-    from_d2(x[(size_t)(ny - 1) * rstride], prev);
+    from_d2(x[(size_t)(ny - 1) * rstride], prev[0]);
     // backward sweep, y descending from ny-2: block b = planes ny-2 - b B - u
     const int nbb = (ny - 1 + B - 1) / B;
     auto issue_b = [&](int b) {
@@ -296,9 +302,9 @@ __device__ __forceinline__ void thomas_line_async(const ThomasArgs& a, int blk, 
                 const double c = ds(st, u);  // c_y / D_y, tabulated with the pivots
                 const double2 v = to_d2(xs(st, u));
                 double2 r;
-                r.x = __dsub_rn(v.x, __dmul_rn(prev.x, c));
-                r.y = __dsub_rn(v.y, __dmul_rn(prev.y, c));
-                prev = r;
+                r.x = __dsub_rn(v.x, __dmul_rn(prev[0].x, c));
+                r.y = __dsub_rn(v.y, __dmul_rn(prev[0].y, c));
+                prev[0] = r;
                 from_d2(x[(size_t)y * rstride], r);
             }
         }
