@@ -145,18 +145,27 @@ int make_dif(int n, prj::DifFft* d, size_t* bytes, int order = 0) {
     return PRJ_OK;
 }
 
-// slot -> wavenumber table of the length-n in-place plan (inverse of its position table)
+// tables of the length-n in-place plan, one after the other: the wavenumber of each slot
+// (n, the inverse of the position table); the pair of each slot (n) and of each folded
+// wavenumber min(kz, n - kz) (n/2 + 1), the pairs numbered in the order of their first slots
+int slot_table_len(int n) { return 2 * n + n / 2 + 1; }
 int make_slot_table(int n, int** d_out, size_t* bytes, int order = 0) {
     prj::DifDev f{};
     const long ntw = prj::dif_plan(n, &f, order);
     if (ntw < 0) return fail(PRJ_ERR_UNSUPPORTED, "no in-place plan for length %d", n);
     std::vector<double2> tw((size_t)ntw);
-    std::vector<int> pos((size_t)n), kz((size_t)n);
+    std::vector<int> pos((size_t)n), tab((size_t)slot_table_len(n), -1);
     prj::dif_fill(f, tw.data(), pos.data());
-    for (int k = 0; k < n; k++) kz[pos[k]] = k;
-    CK(cudaMalloc((void**)d_out, kz.size() * sizeof(int)), "cudaMalloc(slot table)");
-    CK(cudaMemcpy(*d_out, kz.data(), kz.size() * sizeof(int), cudaMemcpyHostToDevice), "cudaMemcpy(slot table)");
-    *bytes += kz.size() * sizeof(int);
+    for (int k = 0; k < n; k++) tab[pos[k]] = k;
+    int next = 0;
+    for (int s = 0; s < n; s++) {
+        int& pair = tab[2 * n + std::min(tab[s], n - tab[s])];
+        if (pair < 0) pair = next++;
+        tab[n + s] = pair;
+    }
+    CK(cudaMalloc((void**)d_out, tab.size() * sizeof(int)), "cudaMalloc(slot table)");
+    CK(cudaMemcpy(*d_out, tab.data(), tab.size() * sizeof(int), cudaMemcpyHostToDevice), "cudaMemcpy(slot table)");
+    *bytes += tab.size() * sizeof(int);
     return PRJ_OK;
 }
 
@@ -427,6 +436,11 @@ int run_mixed_poisson(prj_plan* pl, double* P, cudaStream_t st) {
 
 // z transforms + Thomas: three kernels (split) or one fused kernel
 int run_zsolve(prj_plan* pl, cudaStream_t st) {
+    if (prj::zslab_selected(pl)) {
+        StageTimer tm(pl, prj::kStZSolve, st);
+        CK(prj::launch_zslab(pl, st), "z transform + Thomas (wavenumber on chip)");
+        return PRJ_OK;
+    }
     if (pl->zmode == 3) {
         StageTimer tm(pl, prj::kStZSolve, st);
         const cudaError_t e = prj::launch_zline(pl, st);
@@ -645,7 +659,8 @@ int prj_plan_create(int nx, int nz, int ny, double dx, double dz, const double* 
     {
         int sms = 0;
         if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, pl->device) != cudaSuccess) sms = 0;
-        pl->zmode = z_mode(pl->zd.ok && pl->kz_of_slot, sms > 0 && g.nxh >= 2 * sms);
+        pl->sms = sms;
+        pl->zmode = pl->zmode_default = z_mode(pl->zd.ok && pl->kz_of_slot, sms > 0 && g.nxh >= 2 * sms);
     }
     // pass-plan kernels wherever the length has a plan; the Thomas ring for the
     // mixed-storage solve only (prj_tuning.thomas_ring changes it)
@@ -1138,7 +1153,7 @@ bool x_pass_active(const prj_plan* pl) {
 int prj_plan_schedule(const prj_plan* plan, int mode, int* launches) {
     if (!plan || !launches) return fail(PRJ_ERR_ARG, "NULL argument");
     if (mode == PRJ_MODE_FP64) {
-        const bool one_z = (plan->zmode == 1 || plan->zmode == 2) || (plan->zmode == 3 && prj::zline_supported(plan));
+        const bool one_z = prj::zslab_selected(plan) || (plan->zmode == 1 || plan->zmode == 2) || (plan->zmode == 3 && prj::zline_supported(plan));
         *launches = one_z ? 4 : 6;
     } else {
         // forward x, z transforms of the FP64 and FP32 rows, one Thomas launch, inverse z of both,
@@ -1184,7 +1199,7 @@ int reorder_dif(prj_plan* pl, bool x_axis, int order) {
     cudaDeviceSynchronize();
     prj::DifFft& d = x_axis ? pl->xd : pl->zd;
     const size_t old = (size_t)prj::dif_twiddle_count(d.f) * sizeof(double2) + (size_t)n * sizeof(int) +
-                       (x_axis ? 0 : (size_t)n * sizeof(int));
+                       (x_axis ? 0 : (size_t)slot_table_len(n) * sizeof(int));
     dfree(d.tw);
     dfree(d.pos);
     d = fresh;

@@ -107,7 +107,8 @@ struct prj_plan {
     prj::DifFft xd;               // in-place transform of length fx64.m (x rows)
     prj::DifFft zd;               // in-place transform of length nz (z rows)
     int tz_xd = 1;                // rows per CTA of the in-place x-transform kernels
-    int* kz_of_slot = nullptr;    // z wavenumber held by each slot of zd's output
+    int* kz_of_slot = nullptr;    // z wavenumber held by each slot of zd's output (nz), then the
+                                  // pair (kz, nz - kz) of each slot (nz) and of each kz <= nz/2
     int kxs = 0;                  // spectral rows kx < kxs stored in FP64 (nxh on the FP64 path)
     int kxs_mixed = 0;            // FP64 row count of the mixed path
     int mixed_iters = 1;          // refinement iterations of the mixed path
@@ -121,6 +122,8 @@ struct prj_plan {
     int zfft_rows = 0;            // rows per CTA of the z-transform kernels (0: default rule)
     int zmode = 0;                // z direction: 0 split kernels, 1 fused pipelined, 2 unpipelined,
                                   // 3 one pass-plan kernel per x wavenumber (split where no plan)
+    int zmode_default = 0;        // zmode as the plan was created
+    int sms = 0;                  // SMs of the plan's device
     bool use_pass = true;         // compile-time pass-plan FFT kernels where the length has one
     int thomas_async = -1;        // Thomas lines streamed through a cp.async shared-memory ring:
                                   // -1 for the mixed storage only, 0 never, 1..4 always (ring shape)
@@ -171,6 +174,10 @@ cudaError_t launch_zsolve_pipelined(const prj_plan* pl, int* err_word, cudaStrea
 // z transform + Thomas + inverse z as one kernel per x wavenumber on the pass-plan
 // butterflies (prj_zline.cu); cudaErrorNotSupported when nz has no pass plan
 cudaError_t launch_zline(const prj_plan* pl, cudaStream_t st);
+// the same with a whole x wavenumber on chip, one cluster per wavenumber (prj_zslab.cu), where
+// the plan's z tuning is the default and the wavenumber fits; else cudaErrorNotSupported
+cudaError_t launch_zslab(const prj_plan* pl, cudaStream_t st);
+bool zslab_selected(const prj_plan* pl);  // launch_zslab would run
 bool zline_supported(const prj_plan* pl);  // launch_zline would run (not fall back)
 
 // x transforms with the in-place DIF FFT (prj_xfft.cu); used when pl->xd.ok
