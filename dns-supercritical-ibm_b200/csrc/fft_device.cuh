@@ -109,6 +109,93 @@ __device__ __forceinline__ void dft6(V* a) {
     a[2] = cadd(e2, o2); a[5] = csub(e2, o2);
 }
 
+// R-point DFT of an odd prime R by conjugate pairs: X_k, X_{R-k} = a_0 + sum_r cos(2 pi r k / R)
+// (a_r + a_{R-r}) +- DIR i sum_r sin(2 pi r k / R) (a_r - a_{R-r}), r = 1 .. (R-1)/2
+// cos and sin of 2 pi m / R, 1 <= m <= (R-1)/2
+template <int R>
+__device__ __forceinline__ constexpr double root_cos(int m) {
+    constexpr double c7[] = {0.62348980185873353052500488, -0.2225209339563144042889025, -0.9009688679024191262361023};
+    constexpr double c11[] = {0.84125353283118116886181164, 0.41541501300188642552927414, -0.1423148382732851404437926,
+                              -0.6548607339452850640569250, -0.9594929736144973898903680};
+    constexpr double c13[] = {0.88545602565320989590037552, 0.56806474673115580251180755, 0.12053668025532305334906768,
+                              -0.3546048870425356259696378, -0.7485107481711010986346305, -0.9709418174260520271569822};
+    return R == 7 ? c7[m - 1] : R == 11 ? c11[m - 1] : c13[m - 1];
+}
+template <int R>
+__device__ __forceinline__ constexpr double root_sin(int m) {
+    constexpr double s7[] = {0.78183148246802980870844452, 0.97492791218182360701813168, 0.43388373911755812047576833};
+    constexpr double s11[] = {0.54064081745559758210763595, 0.90963199535451837141171538, 0.98982144188093273237609203,
+                              0.75574957435425828377403584, 0.28173255684142969771141791};
+    constexpr double s13[] = {0.46472317204376854565601533, 0.82298386589365639457961742, 0.99270887409805399280075164,
+                              0.93501624268541482343978459, 0.66312265824079520237678549, 0.23931566428755776714875372};
+    return R == 7 ? s7[m - 1] : R == 11 ? s11[m - 1] : s13[m - 1];
+}
+template <int DIR, int R, typename V>
+__device__ __forceinline__ void dft_prime(V* a) {
+    constexpr int h = (R - 1) / 2;
+    V s[h], d[h];
+#pragma unroll
+    for (int r = 0; r < h; r++) {
+        s[r] = cadd(a[r + 1], a[R - 1 - r]);
+        d[r] = csub(a[r + 1], a[R - 1 - r]);
+    }
+    const V a0 = a[0];
+#pragma unroll
+    for (int r = 0; r < h; r++) a[0] = cadd(a[0], s[r]);
+#pragma unroll
+    for (int k = 1; k <= h; k++) {
+        V e = a0, o = cmk<V>(0, 0);
+#pragma unroll
+        for (int r = 1; r <= h; r++) {
+            const int m = r * k % R;
+            const double c = root_cos<R>(m <= h ? m : R - m);
+            const double n = m <= h ? root_sin<R>(m) : -root_sin<R>(R - m);
+            e = cmk<V>(e.x + c * s[r - 1].x, e.y + c * s[r - 1].y);
+            o = cmk<V>(o.x + n * d[r - 1].x, o.y + n * d[r - 1].y);
+        }
+        o = cmuli<DIR>(o);
+        a[k] = cadd(e, o);
+        a[R - k] = csub(e, o);
+    }
+}
+
+// 9-point DFT: three 3-point DFTs, the twiddles w9^(r k), three 3-point DFTs
+template <int DIR, typename V>
+__device__ __forceinline__ void dft9(V* a) {
+    using T = decltype(V::x);
+#pragma unroll
+    for (int r = 0; r < 3; r++) dft3<DIR>(a[r], a[r + 3], a[r + 6]);
+    const V w1 = cmk<V>(T(0.76604444311897803520239265), T(-0.64278760968653932632264340));
+    const V w2 = cmk<V>(T(0.17364817766693034885171662), T(-0.98480775301220805936674302));
+    const V w4 = cmk<V>(T(-0.9396926207859083840541092), T(-0.34202014332566873304409961));
+    a[4] = DIR < 0 ? cmul(a[4], w1) : cmulc(a[4], w1);
+    a[5] = DIR < 0 ? cmul(a[5], w2) : cmulc(a[5], w2);
+    a[7] = DIR < 0 ? cmul(a[7], w2) : cmulc(a[7], w2);
+    a[8] = DIR < 0 ? cmul(a[8], w4) : cmulc(a[8], w4);
+#pragma unroll
+    for (int k = 0; k < 3; k++) dft3<DIR>(a[3 * k], a[3 * k + 1], a[3 * k + 2]);
+    // output k + 3 q sits at 3 k + q
+    V t;
+    t = a[1]; a[1] = a[3]; a[3] = t;
+    t = a[2]; a[2] = a[6]; a[6] = t;
+    t = a[5]; a[5] = a[7]; a[7] = t;
+}
+
+// 10-point DFT by the prime-factor map n = (5 n1 + 2 n2) mod 10, k = (5 k1 + 6 k2) mod 10: two
+// 5-point DFTs and five 2-point DFTs, no internal twiddles
+template <int DIR, typename V>
+__device__ __forceinline__ void dft10(V* a) {
+    V e[5] = {a[0], a[2], a[4], a[6], a[8]};
+    V o[5] = {a[5], a[7], a[9], a[1], a[3]};
+    dft5<DIR>(e[0], e[1], e[2], e[3], e[4]);
+    dft5<DIR>(o[0], o[1], o[2], o[3], o[4]);
+#pragma unroll
+    for (int k2 = 0; k2 < 5; k2++) {
+        a[6 * k2 % 10] = cadd(e[k2], o[k2]);
+        a[(5 + 6 * k2) % 10] = csub(e[k2], o[k2]);
+    }
+}
+
 // ------------------------------------------------------------ one radix stage
 // i: butterfly index in [0, n/R); k = i mod p.  Inputs src[i + r n/R];
 // outputs dst[(i - k) R + k + r p].
@@ -168,21 +255,28 @@ __device__ __forceinline__ void stage_bfly(const V* __restrict__ src, V* __restr
 #pragma unroll
         for (int r = 0; r < 8; r++) dst[obase + r * p] = a[r];
     } break;
-    default: {
-        // any radix: direct R-point DFT with the stage's root table
-        const V* roots = tw + p * (R - 1);
-        for (int q = 0; q < R; q++) {
-            V acc = cmk<V>(0, 0);
-            for (int r = 0; r < R; r++) {
-                V u = src[i + r * stride];
-                if (r && k) u = DIR < 0 ? cmul(u, w[r - 1]) : cmulc(u, w[r - 1]);
-                const int e = (r * q) % R;
-                acc = cadd(acc, DIR < 0 ? cmul(u, roots[e]) : cmulc(u, roots[e]));
-            }
-            dst[obase + q * p] = acc;
-        }
-    } break;
+    default: break;  // stage_output
     }
+}
+
+// Output q of butterfly i of a radix without a hard-coded kernel: a direct sum with the stage's
+// root table.  One output per thread: a prime radix leaves n / R butterflies of R^2 terms.
+template <int DIR, typename V>
+__device__ __forceinline__ void stage_output(const V* __restrict__ src, V* __restrict__ dst, int n, int R, int p,
+                                             const V* __restrict__ tw, int i, int q) {
+    const int k = i % p, stride = n / R;
+    const V* w = tw + k * (R - 1);
+    const V* roots = tw + p * (R - 1);
+    V acc = src[i];
+    int e = 0;
+    for (int r = 1; r < R; r++) {
+        e += q;
+        if (e >= R) e -= R;
+        V u = src[i + r * stride];
+        if (k) u = DIR < 0 ? cmul(u, w[r - 1]) : cmulc(u, w[r - 1]);
+        acc = cadd(acc, DIR < 0 ? cmul(u, roots[e]) : cmulc(u, roots[e]));
+    }
+    dst[(i - k) * R + k + q * p] = acc;
 }
 
 // Transform `nrows` rows (row stride rs) held in a; b is scratch of the same
@@ -199,10 +293,18 @@ __device__ V* fft_rows(V* a, V* b, int nrows, int rs, const FftDev& f, const V* 
         const int nb = f.n / R;
         const int tot = nb * nrows;
         const V* tws = tw + f.twoff[s];
-        for (int idx = tid; idx < tot; idx += nthr) {
-            const int row = idx / nb;
-            const int i = idx - row * nb;
-            stage_bfly<DIR>(src + row * rs, dst + row * rs, f.n, R, f.p[s], tws, i);
+        if (R == 2 || R == 3 || R == 4 || R == 5 || R == 8) {
+            for (int idx = tid; idx < tot; idx += nthr) {
+                const int row = idx / nb;
+                const int i = idx - row * nb;
+                stage_bfly<DIR>(src + row * rs, dst + row * rs, f.n, R, f.p[s], tws, i);
+            }
+        } else {
+            for (int idx = tid; idx < tot * R; idx += nthr) {
+                const int rq = idx / nb, i = idx - rq * nb;
+                const int row = rq / R, q = rq - row * R;
+                stage_output<DIR>(src + row * rs, dst + row * rs, f.n, R, f.p[s], tws, i, q);
+            }
         }
         __syncthreads();
         V* t = src; src = dst; dst = t;

@@ -9,8 +9,8 @@
 // inverse, time) index k sits at slot pos[k]; consumers read through `pos`.
 //
 // Twiddles per stage: tw[(q - 1) L/R + j] = exp(-2 pi i q j / L), j < L/R,
-// 1 <= q < R.  The inverse transform uses the conjugates.  Radices 2, 3, 4, 5
-// 6 and 8 only; other lengths use the out-of-place path of fft_device.cuh.
+// 1 <= q < R.  The inverse transform uses the conjugates.  Radices 2 .. 11 and 13;
+// lengths with larger prime factors use the out-of-place path of fft_device.cuh.
 #pragma once
 #include "fft_device.cuh"
 
@@ -66,45 +66,56 @@ __device__ __forceinline__ int sidx(int g) {
 // elements per row buffer of n slots with optional padding
 __host__ __device__ inline int padded_len(int n, bool pad) { return pad ? n + (n >> 3) + 1 : n; }
 
-// One butterfly of radix R on elements g0 + r mm (r < R) of buf; w = the stage's twiddles.
-// DIT = false: DFT, then twiddles (decimation in frequency);
-// DIT = true: twiddles, then DFT (its transpose).
-template <int DIR, bool DIT, bool PAD, int R, typename V>
-__device__ __forceinline__ void bfly_r(V* __restrict__ buf, int g0, int mm, int j, const V* __restrict__ w) {
-    V a[R];
-#pragma unroll
-    for (int r = 0; r < R; r++) a[r] = buf[sidx<PAD>(g0 + r * mm)];
-    if (DIT && j) {
-#pragma unroll
-        for (int q = 1; q < R; q++) a[q] = twiddle<DIR>(a[q], w[(q - 1) * mm + j]);
+template <int DIR, int R, typename V>
+__device__ __forceinline__ void dft_r(V* a) {
+    if constexpr (R == 2) dft2<DIR>(a[0], a[1]);
+    else if constexpr (R == 3) dft3<DIR>(a[0], a[1], a[2]);
+    else if constexpr (R == 4) dft4<DIR>(a[0], a[1], a[2], a[3]);
+    else if constexpr (R == 5) dft5<DIR>(a[0], a[1], a[2], a[3], a[4]);
+    else if constexpr (R == 6) dft6<DIR>(a);
+    else if constexpr (R == 8) dft8<DIR>(a);
+    else if constexpr (R == 9) dft9<DIR>(a);
+    else if constexpr (R == 10) dft10<DIR>(a);
+    else {
+        static_assert(R == 7 || R == 11 || R == 13, "radices 2 .. 11 and 13");
+        dft_prime<DIR, R>(a);
     }
-    if (R == 2) dft2<DIR>(a[0], a[1]);
-    else if (R == 3) dft3<DIR>(a[0], a[1], a[2]);
-    else if (R == 4) dft4<DIR>(a[0], a[1], a[2], a[3]);
-    else if (R == 5) dft5<DIR>(a[0], a[1], a[2], a[3], a[4]);
-    else if (R == 6) dft6<DIR>(a);
-    else dft8<DIR>(a);
-    if (!DIT && j) {
-#pragma unroll
-        for (int q = 1; q < R; q++) a[q] = twiddle<DIR>(a[q], w[(q - 1) * mm + j]);
-    }
-#pragma unroll
-    for (int r = 0; r < R; r++) buf[sidx<PAD>(g0 + r * mm)] = a[r];
 }
 
-template <int DIR, bool DIT, bool PAD, typename V>
-__device__ __forceinline__ void bfly(V* __restrict__ buf, int g0, int mm, int R, int j, const V* __restrict__ w) {
-    switch (R) {
-    case 2: bfly_r<DIR, DIT, PAD, 2>(buf, g0, mm, j, w); break;
-    case 3: bfly_r<DIR, DIT, PAD, 3>(buf, g0, mm, j, w); break;
-    case 4: bfly_r<DIR, DIT, PAD, 4>(buf, g0, mm, j, w); break;
-    case 5: bfly_r<DIR, DIT, PAD, 5>(buf, g0, mm, j, w); break;
-    case 6: bfly_r<DIR, DIT, PAD, 6>(buf, g0, mm, j, w); break;
-    case 8: bfly_r<DIR, DIT, PAD, 8>(buf, g0, mm, j, w); break;
-    default:
-        // other radices are planned on the out-of-place Stockham path (fft_device.cuh);
-        // the host never builds a DifDev containing them (dif_supported)
-        break;
+// a[q] *= w1^q with w1 = exp(-+2 pi i j / L) the first row of the stage table (w[j]); the
+// powers come from a product tree of depth <= 4 (a few ulp), so a butterfly loads one
+// twiddle instead of R-1 (the loads were the larger share of the L1 traffic of these kernels)
+template <int DIR, int R, typename V>
+__device__ __forceinline__ void apply_twiddles(V* a, const V* __restrict__ w, int j) {
+    V p[R];
+    p[1] = w[j];
+#pragma unroll
+    for (int q = 2; q < R; q++) p[q] = cmul(p[q / 2], p[q - q / 2]);
+#pragma unroll
+    for (int q = 1; q < R; q++) a[q] = twiddle<DIR>(a[q], p[q]);
+}
+
+// One stage of radix R of the runtime-radix transform: butterflies on elements
+// row rs + b L + j + q mm of buf, nb per row, spans of mm butterflies; w = the stage's twiddles.
+// DIT = false: DFT, then twiddles (decimation in frequency); DIT = true: twiddles, then DFT.
+// Not inlined: each radix is register-allocated on its own.
+template <int DIR, bool DIT, bool PAD, int R, typename V>
+__device__ __noinline__ void stage_r(V* buf, int nrows, int rs, int nb, int mm, FastDiv dnb, FastDiv dmm,
+                                     const V* __restrict__ w) {
+    for (int idx = threadIdx.x; idx < nb * nrows; idx += blockDim.x) {
+        const int row = fdiv(idx, dnb);
+        const int bi = idx - row * nb;
+        const int b = fdiv(bi, dmm);
+        const int j = bi - b * mm;
+        const int g0 = row * rs + b * (mm * R) + j;
+        V a[R];
+#pragma unroll
+        for (int q = 0; q < R; q++) a[q] = buf[sidx<PAD>(g0 + q * mm)];
+        if (DIT && j) apply_twiddles<DIR, R>(a, w, j);
+        dft_r<DIR, R>(a);
+        if (!DIT && j) apply_twiddles<DIR, R>(a, w, j);
+#pragma unroll
+        for (int q = 0; q < R; q++) buf[sidx<PAD>(g0 + q * mm)] = a[q];
     }
 }
 
@@ -115,22 +126,19 @@ __device__ __forceinline__ void bfly(V* __restrict__ buf, int g0, int mm, int R,
 // DIR = +1 it inverts the DIF transform up to the factor n.  Starts and ends
 // with the CTA synchronised.
 template <int DIR, bool DIT, bool PAD, typename V>
-__device__ void inplace_rows(V* buf, int nrows, int rs, const DifDev& f, const V* __restrict__ tw) {
-    const int nthr = blockDim.x, tid = threadIdx.x;
-    const int n = f.n;
+__device__ __forceinline__ void inplace_rows(V* buf, int nrows, int rs, const DifDev& f, const V* __restrict__ tw) {
     for (int t = 0; t < f.nst; t++) {
         const int s = DIT ? f.nst - 1 - t : t;
-        const int R = f.radix[s], L = f.span[s];
-        const int mm = L / R;
-        const int nb = n / R;
-        const V* tws = tw + f.twoff[s];
+        const int R = f.radix[s], nb = f.n / R, mm = f.span[s] / R;
+        const V* w = tw + f.twoff[s];
         const FastDiv dnb = f.nbdiv[s], dmm = f.mmdiv[s];
-        for (int idx = tid; idx < nb * nrows; idx += nthr) {
-            const int row = fdiv(idx, dnb);
-            const int bi = idx - row * nb;
-            const int b = fdiv(bi, dmm);
-            const int j = bi - b * mm;
-            bfly<DIR, DIT, PAD>(buf, row * rs + b * L + j, mm, R, j, tws);
+        switch (R) {
+#define PRJ_STAGE(R_) \
+    case R_: stage_r<DIR, DIT, PAD, R_>(buf, nrows, rs, nb, mm, dnb, dmm, w); break;
+            PRJ_STAGE(2) PRJ_STAGE(3) PRJ_STAGE(4) PRJ_STAGE(5) PRJ_STAGE(6) PRJ_STAGE(7) PRJ_STAGE(8)
+            PRJ_STAGE(9) PRJ_STAGE(10) PRJ_STAGE(11) PRJ_STAGE(13)
+#undef PRJ_STAGE
+        default: break;  // the host plans no other radix here (dif_supported)
         }
         __syncthreads();
     }

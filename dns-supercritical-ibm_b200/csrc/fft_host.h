@@ -39,33 +39,62 @@ inline int pass_orders(int n) {
     return c;
 }
 
-// radix sequence of a length-n transform: the pass plan's radices (in radix order
-// `order`) where one exists, else 8 first, then 4, 2, 3, 5, then any remaining primes;
-// returns the number of stages or -1
+// Fewest passes over the radices 2 .. 11 and 13 (each pass is a round trip through shared
+// memory and a barrier), among those the smallest largest radix (registers), found by trying
+// every multiset in descending order; 0 if n has a larger prime factor.
+inline int short_radices(int n, int most, int left, int* fac) {
+    if (n == 1) return 0;
+    if (left == 0) return -1;
+    static const int radices[] = {13, 11, 10, 9, 8, 7, 6, 5, 4, 3, 2};
+    for (int r : radices) {
+        if (r > most || n % r != 0) continue;
+        const int got = short_radices(n / r, r, left - 1, fac + 1);
+        if (got >= 0) {
+            fac[0] = r;
+            return got + 1;
+        }
+    }
+    return -1;
+}
+
+// radix sequence of a length-n transform: the pass plan's radices (in radix order `order`)
+// where one exists, else the fewest passes; returns the number of stages, or -1 when n has a
+// prime factor above 13.  In the runtime sequence the even radices come first, 8s after them
+// and odd radices last: the last pass's butterflies are R elements apart, and an odd R (or 8,
+// with the padding) spreads them over the banks.
 inline int fft_factorize(int n, int* fac, int cap, int order = 0) {
     const int np = pass_radices(n, fac, cap, order);
     if (np != 0) return np;
-    int nf = 0, m = n;
-    auto push = [&](int r) { if (nf < cap) fac[nf] = r; nf++; };
-    while (m % 8 == 0 && m != 16) { push(8); m /= 8; }
-    while (m % 4 == 0) { push(4); m /= 4; }
-    while (m % 2 == 0) { push(2); m /= 2; }
-    for (int r : {3, 5}) while (m % r == 0) { push(r); m /= r; }
-    for (int r = 7; m > 1; r += 2) {
-        while (m % r == 0) { push(r); m /= r; }
-        if ((long)r * r > m && m > 1) { push(m); m = 1; }
-    }
-    return nf <= cap ? nf : -1;
+    int f[kMaxStages], best[kMaxStages], nb = -1;
+    for (int left = 0; left <= kMaxStages && left <= cap && nb < 0; left++)
+        for (int most = 2; most <= 13 && nb < 0; most++) {
+            const int got = short_radices(n, most, left, f);
+            if (got >= 0) {
+                nb = got;
+                std::memcpy(best, f, sizeof(f));
+            }
+        }
+    if (nb < 0) return -1;
+    auto key = [](int r) { return r % 2 ? 2 : r == 8 ? 1 : 0; };
+    int c = 0;
+    for (int k = 0; k < 3; k++)
+        for (int i = 0; i < nb; i++)
+            if (key(best[i]) == k) fac[c++] = best[i];
+    return nb;
 }
 
-// true when every radix of n has a hard-coded DIF butterfly (2, 3, 4, 5, 6, 8)
+// true when n has an in-place plan: every prime factor at most 13
 inline bool dif_supported(int n) {
-    int fac[64];
-    const int nf = fft_factorize(n, fac, 64);
-    if (nf < 0 || nf > kMaxStages) return false;
-    for (int s = 0; s < nf; s++)
-        if (!(fac[s] == 2 || fac[s] == 3 || fac[s] == 4 || fac[s] == 5 || fac[s] == 6 || fac[s] == 8)) return false;
-    return true;
+    int fac[kMaxStages];
+    return fft_factorize(n, fac, kMaxStages) >= 0;
+}
+
+// true when n is a product of 2, 3 and 5 (the lengths the mixed-precision and distributed
+// paths accept)
+inline bool smooth5(int n) {
+    for (int p : {2, 3, 5})
+        while (n % p == 0) n /= p;
+    return n == 1;
 }
 
 // fills the stage descriptor (radix order `order` where n has a pass plan); returns the

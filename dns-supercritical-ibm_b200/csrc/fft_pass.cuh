@@ -19,19 +19,6 @@
 
 namespace prj {
 
-template <int DIR, int R, typename V>
-__device__ __forceinline__ void dft_r(V* a) {
-    if constexpr (R == 2) dft2<DIR>(a[0], a[1]);
-    else if constexpr (R == 3) dft3<DIR>(a[0], a[1], a[2]);
-    else if constexpr (R == 4) dft4<DIR>(a[0], a[1], a[2], a[3]);
-    else if constexpr (R == 5) dft5<DIR>(a[0], a[1], a[2], a[3], a[4]);
-    else if constexpr (R == 6) dft6<DIR>(a);
-    else {
-        static_assert(R == 8, "radix 2, 3, 4, 5, 6 or 8");
-        dft8<DIR>(a);
-    }
-}
-
 template <int... Rs>
 struct PassList {
     static constexpr int P = sizeof...(Rs);
@@ -77,24 +64,6 @@ __device__ __forceinline__ int pass_slot(int k) {
     }
 }
 
-// a[q] *= w1^q with w1 = exp(-+2 pi i j / L) the first row of the stage table
-// (w[j]); the powers come from a product tree of depth <= 3 (about 3 ulp), so a
-// butterfly loads one twiddle instead of R-1 (the loads were the larger share of
-// the L1 traffic of these kernels)
-template <int DIR, int R, int MM, typename V>
-__device__ __forceinline__ void apply_twiddles(V* a, const V* __restrict__ w, int j) {
-    V p[R];
-    p[1] = w[j];
-    if constexpr (R > 2) p[2] = cmul(p[1], p[1]);
-    if constexpr (R > 3) p[3] = cmul(p[1], p[2]);
-    if constexpr (R > 4) p[4] = cmul(p[2], p[2]);
-    if constexpr (R > 5) p[5] = cmul(p[2], p[3]);
-    if constexpr (R > 6) p[6] = cmul(p[3], p[3]);
-    if constexpr (R > 7) p[7] = cmul(p[3], p[4]);
-#pragma unroll
-    for (int q = 1; q < R; q++) a[q] = twiddle<DIR>(a[q], p[q]);
-}
-
 // One pass s of nrows rows held in shared memory (row stride rs, padded slots):
 // DIT = false: DFT then twiddles; DIT = true: twiddles then DFT.
 template <int DIR, bool DIT, class PL, int S, typename V>
@@ -108,9 +77,9 @@ __device__ __forceinline__ void pass_shared(V* buf, int nrows, int rs, const V* 
         V a[R];
 #pragma unroll
         for (int q = 0; q < R; q++) a[q] = buf[sidx<true>(g0 + q * mm)];
-        if (DIT && mm > 1 && j) apply_twiddles<DIR, R, mm>(a, tws, j);
+        if (DIT && mm > 1 && j) apply_twiddles<DIR, R>(a, tws, j);
         dft_r<DIR, R>(a);
-        if (!DIT && mm > 1 && j) apply_twiddles<DIR, R, mm>(a, tws, j);
+        if (!DIT && mm > 1 && j) apply_twiddles<DIR, R>(a, tws, j);
 #pragma unroll
         for (int q = 0; q < R; q++) buf[sidx<true>(g0 + q * mm)] = a[q];
     }
@@ -147,7 +116,7 @@ __device__ __forceinline__ void dif_first_pass(V* buf, int nrows, int rs, const 
 #pragma unroll
         for (int q = 0; q < R; q++) a[q] = ld(row, j + q * mm);
         dft_r<DIR, R>(a);
-        if (mm > 1 && j) apply_twiddles<DIR, R, mm>(a, tw, j);
+        if (mm > 1 && j) apply_twiddles<DIR, R>(a, tw, j);
 #pragma unroll
         for (int q = 0; q < R; q++) buf[sidx<true>(row * rs + j + q * mm)] = a[q];
     }
@@ -196,7 +165,7 @@ __device__ __forceinline__ void dit_last_pass(const V* buf, int nrows, int rs, c
         V a[R];
 #pragma unroll
         for (int q = 0; q < R; q++) a[q] = buf[sidx<true>(row * rs + j + q * mm)];
-        if (mm > 1 && j) apply_twiddles<DIR, R, mm>(a, tw, j);
+        if (mm > 1 && j) apply_twiddles<DIR, R>(a, tw, j);
         dft_r<DIR, R>(a);
 #pragma unroll
         for (int q = 0; q < R; q++) st(row, j + q * mm, a[q]);
@@ -264,6 +233,6 @@ inline bool same_radices(const DifDev& f) {
 // a multiple of 8, so every row starts on a padding boundary and the passes of
 // consecutive rows see the same bank pattern; the +8 offsets consecutive rows by
 // one bank group for the row-fastest split and load phases.
-__host__ __device__ constexpr int pass_row_stride(int m) { return m + 8; }
+__host__ __device__ constexpr int pass_row_stride(int m) { return (m + 7) / 8 * 8 + 8; }
 
 }  // namespace prj

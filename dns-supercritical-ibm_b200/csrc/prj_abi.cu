@@ -150,12 +150,16 @@ int make_dif(int n, prj::DifFft* d, size_t* bytes, int order = 0) {
 // wavenumber min(kz, n - kz) (n/2 + 1), the pairs numbered in the order of their first slots
 int slot_table_len(int n) { return 2 * n + n / 2 + 1; }
 int make_slot_table(int n, int** d_out, size_t* bytes, int order = 0) {
-    prj::DifDev f{};
-    const long ntw = prj::dif_plan(n, &f, order);
-    if (ntw < 0) return fail(PRJ_ERR_UNSUPPORTED, "no in-place plan for length %d", n);
-    std::vector<double2> tw((size_t)ntw);
     std::vector<int> pos((size_t)n), tab((size_t)slot_table_len(n), -1);
-    prj::dif_fill(f, tw.data(), pos.data());
+    if (prj::dif_supported(n)) {
+        prj::DifDev f{};
+        const long ntw = prj::dif_plan(n, &f, order);
+        if (ntw < 0) return fail(PRJ_ERR_UNSUPPORTED, "no in-place plan for length %d", n);
+        std::vector<double2> tw((size_t)ntw);
+        prj::dif_fill(f, tw.data(), pos.data());
+    } else {  // the out-of-place transforms leave natural order
+        for (int k = 0; k < n; k++) pos[k] = k;
+    }
     for (int k = 0; k < n; k++) tab[pos[k]] = k;
     int next = 0;
     for (int s = 0; s < n; s++) {
@@ -413,7 +417,7 @@ int run_mixed_solve(prj_plan* pl, const double* Uh, const double* Vh, const doub
 }
 
 int mixed_supported(const prj_plan* pl) {
-    if ((pl->zmode != 0 && pl->zmode != 3) || !pl->xd.ok)
+    if ((pl->zmode != 0 && pl->zmode != 3) || !prj::smooth5(pl->fx64.m) || !prj::smooth5(pl->g.nz))
         return fail(PRJ_ERR_UNSUPPORTED, "the mixed-precision path needs in-place plans for nx/2 and nz (radices 2, 3, 4, 5, 8)");
     return PRJ_OK;
 }
@@ -434,6 +438,13 @@ int run_mixed_poisson(prj_plan* pl, double* P, cudaStream_t st) {
     return run_mixed_core(pl, nullptr, nullptr, nullptr, nullptr, pl->mix_b, pl->mix_r, P, st);
 }
 
+// three z kernels: by the tuning, and by default for lengths with a prime factor above 5 (the
+// runtime-radix kernel per wavenumber, k_zsolve_pipe, took 346 us for 68 wavenumbers of 60
+// planes at nz = 77, where the three take 40)
+bool split_z(const prj_plan* pl) {
+    return pl->zmode == 0 || pl->zmode == 3 || (pl->zmode == 1 && pl->zmode_default == 1 && pl->z_planes == 0 && pl->z_stages == 0);
+}
+
 // z transforms + Thomas: three kernels (split) or one fused kernel
 int run_zsolve(prj_plan* pl, cudaStream_t st) {
     if (prj::zslab_selected(pl)) {
@@ -449,7 +460,7 @@ int run_zsolve(prj_plan* pl, cudaStream_t st) {
             return PRJ_OK;
         }
     }
-    if (pl->zmode == 0 || pl->zmode == 3) {
+    if (split_z(pl)) {
         {
             StageTimer tm(pl, prj::kStZfftFwd, st);
             CK(prj::launch_zfft(pl, -1, st), "z transform");
@@ -655,12 +666,12 @@ int prj_plan_create(int nx, int nz, int ny, double dx, double dz, const double* 
     if ((rc = make_cfft<double>(nz, &pl->fz64.f, &pl->fz64.tw, &bytes))) return bail(rc);
     if ((rc = make_dif(pl->fx64.m, &pl->xd, &bytes))) return bail(rc);
     if ((rc = make_dif(nz, &pl->zd, &bytes))) return bail(rc);
-    if (pl->zd.ok && (rc = make_slot_table(nz, &pl->kz_of_slot, &bytes))) return bail(rc);
+    if ((rc = make_slot_table(nz, &pl->kz_of_slot, &bytes))) return bail(rc);
     {
         int sms = 0;
         if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, pl->device) != cudaSuccess) sms = 0;
         pl->sms = sms;
-        pl->zmode = pl->zmode_default = z_mode(pl->zd.ok && pl->kz_of_slot, sms > 0 && g.nxh >= 2 * sms);
+        pl->zmode = pl->zmode_default = z_mode(prj::smooth5(nz), sms > 0 && g.nxh >= 2 * sms);
     }
     // pass-plan kernels wherever the length has a plan; the Thomas ring for the
     // mixed-storage solve only (prj_tuning.thomas_ring changes it)
@@ -1144,16 +1155,14 @@ int prj_poisson_mixed(prj_plan* plan, double* d_P, void* stream) {
     return run_mixed_poisson(plan, d_P, (cudaStream_t)stream);
 }
 
-// true when the x transforms run the pass-plan kernels (even nx, m = nx/2 with a plan)
-bool x_pass_active(const prj_plan* pl) {
-    int fac[8];
-    return pl->use_pass && pl->fx64.even && pl->xd.ok && prj::pass_radices(pl->fx64.m, fac, 8) > 0;
-}
+// true when the x transforms run the tiled kernels (even nx with an in-place plan), which also
+// form the mixed path's residual
+bool x_pass_active(const prj_plan* pl) { return pl->use_pass && pl->fx64.even && pl->xd.ok; }
 
 int prj_plan_schedule(const prj_plan* plan, int mode, int* launches) {
     if (!plan || !launches) return fail(PRJ_ERR_ARG, "NULL argument");
     if (mode == PRJ_MODE_FP64) {
-        const bool one_z = prj::zslab_selected(plan) || (plan->zmode == 1 || plan->zmode == 2) || (plan->zmode == 3 && prj::zline_supported(plan));
+        const bool one_z = prj::zslab_selected(plan) || !split_z(plan) || (plan->zmode == 3 && prj::zline_supported(plan));
         *launches = one_z ? 4 : 6;
     } else {
         // forward x, z transforms of the FP64 and FP32 rows, one Thomas launch, inverse z of both,
@@ -1221,7 +1230,7 @@ int prj_plan_set_tuning(prj_plan* plan, const prj_tuning* t) {
     if (!pow2(t->x_rows)) return fail(PRJ_ERR_ARG, "x_rows=%d must be a power of two in [1, 16]", t->x_rows);
     if (t->z_rows != 0 && !pow2(t->z_rows)) return fail(PRJ_ERR_ARG, "z_rows=%d must be 0 or a power of two in [1, 16]", t->z_rows);
     if (t->z_mode < 0 || t->z_mode > 3) return fail(PRJ_ERR_ARG, "z_mode=%d must be 0, 1, 2 or 3", t->z_mode);
-    if ((t->z_mode == 0 || t->z_mode == 3) && !(plan->zd.ok && plan->kz_of_slot))
+    if ((t->z_mode == 0 || t->z_mode == 3) && !prj::smooth5(plan->g.nz))
         return fail(PRJ_ERR_UNSUPPORTED, "no in-place z plan for nz=%d", plan->g.nz);
     if (t->z_planes < 0 || t->z_planes > 64) return fail(PRJ_ERR_ARG, "z_planes=%d must lie in [0, 64]", t->z_planes);
     if (t->z_stages != 0 && (t->z_stages < 2 || t->z_stages > (t->z_mode == 1 ? 8 : 4)))

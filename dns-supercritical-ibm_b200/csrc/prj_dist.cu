@@ -31,7 +31,7 @@ int dist_check(const prj_plan* pl, int y0, int y1) {
     int fac[8];
     if (!pl->use_pass || !pl->zd.ok || !pl->kz_of_slot || prj::pass_radices(pl->g.nz, fac, 8) <= 0)
         return record_error(PRJ_ERR_UNSUPPORTED, "prj_dist: needs a z length with a compile-time pass plan");
-    if (!pl->xd.ok)
+    if (!prj::smooth5(pl->fx64.m))
         return record_error(PRJ_ERR_UNSUPPORTED, "prj_dist: needs an x length of radices 2, 3, 4, 5, 6, 8");
     return PRJ_OK;
 }

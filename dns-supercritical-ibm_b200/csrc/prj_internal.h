@@ -16,7 +16,7 @@
 namespace prj {
 
 // In-place DIF transform of one length (fft_dif.cuh): descriptor and device tables.
-// `ok` is false when a radix has no hard-coded butterfly; the out-of-place
+// `ok` is false when the length has a prime factor above 13; the out-of-place
 // Stockham kernels serve those lengths.
 struct DifFft {
     bool ok = false;
@@ -199,7 +199,7 @@ int choose_tz_xd(int m, bool even);
 int choose_tz_xp(int m);                 // rows per CTA of the pass-plan x kernels
 size_t pass_x_smem(int m, int tz);       // their shared memory
 
-// z direction as separate kernels (prj_zsplit.cu); need pl->zd.ok and pl->kz_of_slot
+// z direction as separate kernels (prj_zsplit.cu)
 cudaError_t launch_zfft(const prj_plan* pl, int dir, cudaStream_t st, YRange yr = YRange{});
 cudaError_t launch_thomas(const prj_plan* pl, cudaStream_t st);
 // Thomas sweeps of the lines kx0 .. kx0+rows-1 held in X as [y][kx - kx0][z] (FP64)

@@ -11,6 +11,7 @@
 // CTAs fit on an SM.  Loads and stores of P and u_hat are one element per
 // thread along x (fully coalesced).
 #include "fft_dif.cuh"
+#include "fft_host.h"
 #include "fft_pass.cuh"
 #include "prj_internal.h"
 #include "xfft_tiles.cuh"
@@ -226,13 +227,13 @@ __global__ void __launch_bounds__(256, PRJ_FFT_MINB) k_bwd_xd(const XArgs a) {
 
 // k_fwd_xp / k_bwd_xp: one CTA per tile of the pass-plan x transforms (xfft_tiles.cuh)
 template <int SRC, class PL>
-__global__ void __launch_bounds__(kPassThreads, PRJ_PASS_MINB) k_fwd_xp(const XArgs a) {
+__global__ void __launch_bounds__(x_threads(PL::n), x_minb(PL::n)) k_fwd_xp(const XArgs a) {
     extern __shared__ __align__(16) unsigned char sm[];
     fwd_xp_tile<SRC, PL>(a, sm, blockIdx.x, blockIdx.y);
 }
 
 template <class PL>
-__global__ void __launch_bounds__(kPassThreads, PRJ_PASS_MINB) k_bwd_xp(const XArgs a) {
+__global__ void __launch_bounds__(x_threads(PL::n), x_minb(PL::n)) k_bwd_xp(const XArgs a) {
     extern __shared__ __align__(16) unsigned char sm[];
     bwd_xp_tile<PL>(a, sm, blockIdx.x, blockIdx.y, gridDim.x);
 }
@@ -244,7 +245,7 @@ XArgs make_args(const prj_plan* pl) {
     a.m = pl->fx64.m; a.even = pl->fx64.even;
     a.tz = pl->tz_xd;
     a.rs = a.even ? a.m + 1 : a.m;
-    a.f = pl->xd.f; a.tw = pl->xd.tw; a.pos = pl->xd.pos; a.post = pl->fx64.post;
+    a.f = pl->xd.f; a.mdiv = make_fastdiv((unsigned)a.m); a.tw = pl->xd.tw; a.pos = pl->xd.pos; a.post = pl->fx64.post;
     a.inv_dx = 1.0 / g.dx; a.inv_dz = 1.0 / g.dz;
     a.X = pl->spec;
     a.X32 = pl->spec32;
@@ -282,10 +283,12 @@ cudaError_t allow_smem(K kernel, size_t bytes) {
 int bwd_tiles_per_plane(const prj_plan* pl) { return (pl->g.nz + pl->tz_xp - 1) / pl->tz_xp; }
 
 // rows per CTA of the pass-plan x kernels: a power of two up to 16 whose padded rows
-// (stride pass_row_stride(m)) fit 32 KB, so that 6 CTAs share an SM
+// (stride pass_row_stride(m)) fit 32 KB, so that 6 CTAs share an SM; for the plans from m = 768,
+// where that is two rows, 64 KB and 256 threads
 int choose_tz_xp(int m) {
     int tz = 16;
-    while (tz > 1 && (size_t)padded_len(tz * pass_row_stride(m), true) * sizeof(double2) > 32 * 1024) tz /= 2;
+    const size_t most = (size_t)(pass_orders(m) > 0 ? x_threads(m) / kPassThreads : 1) * 32 * 1024;
+    while (tz > 1 && (size_t)padded_len(tz * pass_row_stride(m), true) * sizeof(double2) > most) tz /= 2;
     return tz;
 }
 
@@ -313,13 +316,13 @@ cudaError_t launch_fwd_xp_pl(const XArgs& a, FwdSource src, const dim3& grid, cu
     cudaError_t e;
     if (src == FwdSource::Pressure) {
         if ((e = allow_smem(k_fwd_xp<0, PL>, smem)) != cudaSuccess) return e;
-        k_fwd_xp<0, PL><<<grid, kPassThreads, smem, st>>>(a);
+        k_fwd_xp<0, PL><<<grid, x_threads(PL::n), smem, st>>>(a);
     } else if (src == FwdSource::Residual) {
         if ((e = allow_smem(k_fwd_xp<3, PL>, smem)) != cudaSuccess) return e;
-        k_fwd_xp<3, PL><<<grid, kPassThreads, smem, st>>>(a);
+        k_fwd_xp<3, PL><<<grid, x_threads(PL::n), smem, st>>>(a);
     } else {
         if ((e = allow_smem(k_fwd_xp<1, PL>, smem)) != cudaSuccess) return e;
-        k_fwd_xp<1, PL><<<grid, kPassThreads, smem, st>>>(a);
+        k_fwd_xp<1, PL><<<grid, x_threads(PL::n), smem, st>>>(a);
     }
     return cudaGetLastError();
 }
@@ -329,15 +332,15 @@ cudaError_t launch_bwd_xp_pl(const XArgs& a, const dim3& grid, cudaStream_t st) 
     const size_t smem = pass_smem_bytes(a);
     cudaError_t e = allow_smem(k_bwd_xp<PL>, smem);
     if (e != cudaSuccess) return e;
-    k_bwd_xp<PL><<<grid, kPassThreads, smem, st>>>(a);
+    k_bwd_xp<PL><<<grid, x_threads(PL::n), smem, st>>>(a);
     return cudaGetLastError();
 }
 
-// pass-plan x kernels for even nx whose half length has a pass plan built with the
-// same radices; cudaErrorNotSupported otherwise (the caller uses the runtime-radix kernels)
+// x kernels for even nx: the half length's compile-time pass plan, or the runtime radices;
+// cudaErrorNotSupported otherwise (the caller uses k_fwd_xd / k_bwd_xd)
 cudaError_t launch_xpass(const prj_plan* pl, bool fwd, FwdSource src, XArgs a, int ny_launch, cudaStream_t st) {
-    if (!pl->use_pass || !a.even) return cudaErrorNotSupported;
     a.tz = pl->tz_xp;
+    if (!pl->use_pass || !a.even || !pl->xd.ok || pass_smem_bytes(a) > (size_t)200 * 1024) return cudaErrorNotSupported;
     const dim3 grid((pl->g.nz + a.tz - 1) / a.tz, ny_launch);
 #define PRJ_X_CASE(N, ...)                                                                          \
     if (a.m == N && same_radices<PassList<__VA_ARGS__>>(pl->xd.f)) {                                \
@@ -346,7 +349,7 @@ cudaError_t launch_xpass(const prj_plan* pl, bool fwd, FwdSource src, XArgs a, i
     }
     PRJ_PASS_ALL(PRJ_X_CASE)
 #undef PRJ_X_CASE
-    return cudaErrorNotSupported;
+    return fwd ? launch_fwd_xp_pl<RuntimePlan>(a, src, grid, st) : launch_bwd_xp_pl<RuntimePlan>(a, grid, st);
 }
 
 }  // namespace
@@ -359,7 +362,9 @@ cudaError_t launch_fwd_xd(const prj_plan* pl, FwdSource src, const double* P, co
     a.Bout = bout;
     a.P = P; a.Uh = Uh; a.Vh = Vh; a.Wh = Wh; a.inv_dy_p = pl->t.inv_dy_p;
     if (sc) { a.inv_dt = sc->inv_dt; a.vbot = sc->wall[1]; a.vtop = sc->wall[4]; }
-    if (src == FwdSource::Divergence || (aligned16(P) && aligned16(bout))) {
+    const bool al = src == FwdSource::Divergence ? aligned16(Uh) && aligned16(Vh) && aligned16(Wh) && aligned16(bout)
+                                                 : aligned16(P) && aligned16(bout);
+    if (al) {
         const cudaError_t e = launch_xpass(pl, true, src, a, yr.y1 - yr.y0, st);
         if (e != cudaErrorNotSupported) return e;
     }

@@ -6,8 +6,9 @@
 // inverse split (scaled) -> DIT passes -> P rows.  The kernels k_fwd_xp / k_bwd_xp
 // (prj_xfft.cu) run one tile per CTA; the persistent batch kernel (prj_batchk.cu)
 // runs tiles of many cases from a work queue with the same code, so both give the
-// same bits.  m = nx/2 has a compile-time plan PL; rows sit at stride
-// pass_row_stride(m) in shared memory (`sm`, 16-byte aligned).
+// same bits.  m = nx/2 has a compile-time plan PL, or the runtime
+// radices of fft_dif.cuh (RuntimePlan); rows sit at stride pass_row_stride(m) in shared
+// memory (`sm`, 16-byte aligned).
 #pragma once
 #include "cp_async.cuh"
 #include "fft_dif.cuh"
@@ -33,6 +34,7 @@ __device__ __forceinline__ size_t hidx_d(int nx, int nz, int i, int j, int k) {
 struct XArgs {
     int nx, nz, ny, nh, m, tz, rs, even;
     DifDev f;
+    FastDiv mdiv;    // m (RuntimePlan)
     const double2* tw;
     const int* pos;
     const double2* post;
@@ -80,6 +82,36 @@ __device__ __forceinline__ double2 spec_load(const XArgs& a, int y, int kx, int 
 // the current tile computes: the forward's P rows z0 .. z0+nr-1 of plane y, contiguous in
 // P, as S[r m + e]; the inverse's spectrum X[y][k][z0 + r] as S[k tz + r], k = 0 .. m.
 
+// threads per CTA and resident CTAs per SM of the one-tile kernels (0: RuntimePlan)
+__host__ __device__ constexpr int x_threads(int m) { return m >= 768 ? 256 : kPassThreads; }
+__host__ __device__ constexpr int x_minb(int m) { return x_threads(m) == kPassThreads ? PRJ_PASS_MINB : PRJ_PASS_MINB / 2; }
+
+// lengths without a compile-time plan
+struct RuntimePlan {
+    static constexpr int n = 0, P = 0;
+};
+template <class PL>
+__device__ __forceinline__ int x_len(const XArgs& a) {
+    if constexpr (PL::n > 0) return PL::n;
+    else return a.m;
+}
+template <class PL>
+__device__ __forceinline__ int x_row(const XArgs& a, int idx) {  // idx / m
+    if constexpr (PL::n > 0) return idx / PL::n;
+    else return fdiv(idx, a.mdiv);
+}
+template <class PL>
+__device__ __forceinline__ int x_slot(const XArgs& a, int k) {
+    if constexpr (PL::n > 0) return pass_slot<PL>(k);
+    else return a.pos[k];
+}
+// every forward pass of nr rows, a barrier after each
+template <class PL>
+__device__ __forceinline__ void x_forward(const XArgs& a, double2* A, int nr, int rs) {
+    if constexpr (PL::n > 0) dif_passes_shared<-1, PL, 0, PL::P>(A, nr, rs, a.tw);
+    else inplace_rows<-1, false, true>(A, nr, rs, a.f, a.tw);
+}
+
 // fwd_xp_tile: source (P, or the divergence of u_hat) -> packed complex -> DIF
 // passes -> split X_k, X_{m-k} -> transposed store.  SRC 0 reads P in the first
 // pass; SRC 1 stages the divergence in shared memory first; SRC 2 reads P from S
@@ -90,7 +122,7 @@ template <int SRC, class PL, class Hook = NoHook>
 __device__ __forceinline__ void fwd_xp_tile(const XArgs& a, unsigned char* sm, int bx, int by,
                                             const double2* S = nullptr, Hook after_first = Hook{}) {
     double2* A = reinterpret_cast<double2*>(sm);
-    constexpr int m = PL::n, nx = 2 * m, rs = pass_row_stride(m);
+    const int m = x_len<PL>(a), nx = 2 * m, rs = pass_row_stride(m);
     const int tid = threadIdx.x, nthr = blockDim.x;
     const int y = a.y0 + by, z0 = bx * a.tz;
     const int nr = min(a.tz, a.nz - z0);
@@ -118,7 +150,7 @@ __device__ __forceinline__ void fwd_xp_tile(const XArgs& a, unsigned char* sm, i
             for (int u = 0; u < kDivUnroll; u++) {
                 const int idx = base + u * nthr + lane;
                 const bool in = idx < total;
-                const int r = in ? idx / m : 0, e = in ? idx - r * m : 0;
+                const int r = in ? x_row<PL>(a, idx) : 0, e = in ? idx - r * m : 0;
                 const int z = z0 + r, zp = (z + 1 == a.nz) ? 0 : z + 1;
                 const size_t c0 = (size_t)(y + 1) * hplane + (size_t)(z + 1) * hrow + 1;
                 const size_t cz = (size_t)(y + 1) * hplane + (size_t)(zp + 1) * hrow + 1;
@@ -136,7 +168,7 @@ __device__ __forceinline__ void fwd_xp_tile(const XArgs& a, unsigned char* sm, i
             for (int u = 0; u < kDivUnroll; u++) {
                 const int idx = base + u * nthr + lane;
                 const bool in = idx < total;
-                const int r = in ? idx / m : 0, e = in ? idx - r * m : 0;
+                const int r = in ? x_row<PL>(a, idx) : 0, e = in ? idx - r * m : 0;
                 const int z = z0 + r, zp = (z + 1 == a.nz) ? 0 : z + 1;
                 const size_t c0 = (size_t)(y + 1) * hplane + (size_t)(z + 1) * hrow + 1;
                 const size_t cz = (size_t)(y + 1) * hplane + (size_t)(zp + 1) * hrow + 1;
@@ -174,7 +206,7 @@ __device__ __forceinline__ void fwd_xp_tile(const XArgs& a, unsigned char* sm, i
             }
         }
         __syncthreads();
-        dif_passes_shared<-1, PL, 0, PL::P>(A, nr, rs, tw);
+        x_forward<PL>(a, A, nr, rs);
     } else if (SRC == 3) {
         // the residual at the x pair (2e, 2e+1) of row z0 + r, as packed complex element e:
         // P, B and the z and wall-normal neighbour rows read as aligned pairs, the x
@@ -186,7 +218,7 @@ __device__ __forceinline__ void fwd_xp_tile(const XArgs& a, unsigned char* sm, i
         const size_t plane = (size_t)nz * nx;
         const int total = nr * m;
         for (int idx = tid; idx < total; idx += nthr) {
-            const int r = idx / m, e = idx - r * m;
+            const int r = x_row<PL>(a, idx), e = idx - r * m;
             const int z = z0 + r, zp = (z + 1 == nz) ? 0 : z + 1, zm = (z == 0) ? nz - 1 : z - 1;
             const size_t row = (size_t)y * plane + (size_t)z * nx;
             const double* p0 = a.P + row;
@@ -206,25 +238,46 @@ __device__ __forceinline__ void fwd_xp_tile(const XArgs& a, unsigned char* sm, i
             A[sidx<true>(r * rs + e)] = make_double2(r0, r1);
         }
         __syncthreads();
-        dif_passes_shared<-1, PL, 0, PL::P>(A, nr, rs, tw);
+        x_forward<PL>(a, A, nr, rs);
     } else {
         const double2* src = reinterpret_cast<const double2*>(a.P) + ((size_t)y * a.nz + z0) * m;
         double2* bout = a.Bout ? reinterpret_cast<double2*>(a.Bout) + ((size_t)y * a.nz + z0) * m : nullptr;
-        if constexpr (SRC == 2) {
-            dif_first_pass<-1, PL>(A, nr, rs, tw, [&](int r, int e) { return S[(size_t)r * m + e]; });
+        if constexpr (PL::n == 0) {
+            static_assert(SRC != 2, "the batch kernel has compile-time plans");
+            for (int base = tid; base < nr * m; base += kUnroll * nthr) {
+                double2 v[kUnroll];
+#pragma unroll
+                for (int u = 0; u < kUnroll; u++)
+                    if (base + u * nthr < nr * m) v[u] = src[base + u * nthr];
+#pragma unroll
+                for (int u = 0; u < kUnroll; u++) {
+                    const int idx = base + u * nthr;
+                    if (idx < nr * m) {
+                        const int r = x_row<PL>(a, idx);
+                        if (bout) bout[idx] = v[u];
+                        A[sidx<true>(r * rs + idx - r * m)] = v[u];
+                    }
+                }
+            }
+            __syncthreads();
+            x_forward<PL>(a, A, nr, rs);
         } else {
-            dif_first_pass<-1, PL>(A, nr, rs, tw, [&](int r, int e) {
-                const double2 v = src[(size_t)r * m + e];
-                if (bout) bout[(size_t)r * m + e] = v;
-                return v;
-            });
+            if constexpr (SRC == 2) {
+                dif_first_pass<-1, PL>(A, nr, rs, tw, [&](int r, int e) { return S[(size_t)r * m + e]; });
+            } else {
+                dif_first_pass<-1, PL>(A, nr, rs, tw, [&](int r, int e) {
+                    const double2 v = src[(size_t)r * m + e];
+                    if (bout) bout[(size_t)r * m + e] = v;
+                    return v;
+                });
+            }
+            __syncthreads();
+            after_first();
+            dif_passes_shared<-1, PL, 1, PL::P>(A, nr, rs, tw);
         }
-        __syncthreads();
-        after_first();
-        dif_passes_shared<-1, PL, 1, PL::P>(A, nr, rs, tw);
     }
     // split: X_k = E_k + W^k O_k, X_{m-k} = conj(E_k) + W^{m-k} conj(O_k); row index fastest
-    constexpr int half = m / 2;
+    const int half = m / 2;
     for (int idx = tid; idx < nr * (half + 1); idx += nthr) {
         const int k = idx / nr, r = idx - k * nr;
         const int base = r * rs;
@@ -235,8 +288,8 @@ __device__ __forceinline__ void fwd_xp_tile(const XArgs& a, unsigned char* sm, i
             spec_store(a, y, m, z, make_double2(c.x - c.y, 0.0));
         } else {
             const int kk = m - k;
-            const double2 zk = A[sidx<true>(base + pass_slot<PL>(k))];
-            const double2 zm = cconj(A[sidx<true>(base + pass_slot<PL>(kk))]);
+            const double2 zk = A[sidx<true>(base + x_slot<PL>(a, k))];
+            const double2 zm = cconj(A[sidx<true>(base + x_slot<PL>(a, kk))]);
             const double2 e = cscale(cadd(zk, zm), 0.5);
             const double2 d = csub(zk, zm);
             const double2 o = make_double2(0.5 * d.y, -0.5 * d.x);
@@ -256,7 +309,7 @@ template <class PL, bool EXTRAS = true, bool STAGED = false, class Hook = NoHook
 __device__ __forceinline__ void bwd_xp_tile(const XArgs& a, unsigned char* sm, int bx, int by, int tiles_per_plane,
                                             const double2* S = nullptr, Hook after_split = Hook{}) {
     double2* A = reinterpret_cast<double2*>(sm);
-    constexpr int m = PL::n, rs = pass_row_stride(m), half = m / 2;
+    const int m = x_len<PL>(a), rs = pass_row_stride(m), half = m / 2;
     const int tid = threadIdx.x, nthr = blockDim.x;
     const int y = a.y0 + by, z0 = bx * a.tz;
     const int nr = min(a.tz, a.nz - z0);
@@ -293,25 +346,37 @@ __device__ __forceinline__ void bwd_xp_tile(const XArgs& a, unsigned char* sm, i
                 const double2 xk = xa[u], xkk = xb[u];
                 const double2 e1 = cadd(xk, cconj(xkk));
                 const double2 o1 = cmulc(csub(xk, cconj(xkk)), a.post[k]);
-                A[sidx<true>(base + pass_slot<PL>(k))] = cscale(make_double2(e1.x - o1.y, e1.y + o1.x), s);
+                A[sidx<true>(base + x_slot<PL>(a, k))] = cscale(make_double2(e1.x - o1.y, e1.y + o1.x), s);
                 if (kk != k) {
                     const double2 e2 = cadd(xkk, cconj(xk));
                     const double2 o2 = cmulc(csub(xkk, cconj(xk)), a.post[kk]);
-                    A[sidx<true>(base + pass_slot<PL>(kk))] = cscale(make_double2(e2.x - o2.y, e2.y + o2.x), s);
+                    A[sidx<true>(base + x_slot<PL>(a, kk))] = cscale(make_double2(e2.x - o2.y, e2.y + o2.x), s);
                 }
             }
         }
     }
     __syncthreads();
     after_split();
-    dit_passes_shared<+1, PL, PL::P - 1, 0>(A, nr, rs, a.tw);
+    // the last pass hands its values to st(r, e, value)
+    auto inverse = [&](auto st) {
+        if constexpr (PL::n > 0) {
+            dit_passes_shared<+1, PL, PL::P - 1, 0>(A, nr, rs, a.tw);
+            dit_last_pass<+1, PL>(A, nr, rs, a.tw, st);
+        } else {
+            inplace_rows<+1, true, true>(A, nr, rs, a.f, a.tw);
+            for (int idx = tid; idx < nr * m; idx += nthr) {
+                const int r = x_row<PL>(a, idx), e = idx - r * m;
+                st(r, e, A[sidx<true>(r * rs + e)]);
+            }
+        }
+    };
     double2* out = reinterpret_cast<double2*>(a.Pout) + ((size_t)y * a.nz + z0) * m;
     double sq0 = 0.0, sq1 = 0.0, ps = 0.0;
     if constexpr (!EXTRAS) {
-        dit_last_pass<+1, PL>(A, nr, rs, a.tw, [&](int r, int e, double2 v) { out[(size_t)r * m + e] = v; });
+        inverse([&](int r, int e, double2 v) { out[(size_t)r * m + e] = v; });
         return;
     }
-    dit_last_pass<+1, PL>(A, nr, rs, a.tw, [&](int r, int e, double2 v) {
+    inverse([&](int r, int e, double2 v) {
         double2* o = out + (size_t)r * m + e;
         if (a.accum) {
             const double2 old = *o;
@@ -327,7 +392,7 @@ __device__ __forceinline__ void bwd_xp_tile(const XArgs& a, unsigned char* sm, i
     });
     if (a.psum) {
         // the tile's sum in a fixed order (per thread, then warp butterfly, then warps in order)
-        __shared__ double wsum[kPassThreads / 32];
+        __shared__ double wsum[8];  // warps of at most 256 threads
         for (int o = 16; o > 0; o >>= 1) ps += __shfl_xor_sync(0xffffffffu, ps, o);
         if ((tid & 31) == 0) wsum[tid >> 5] = ps;
         __syncthreads();
