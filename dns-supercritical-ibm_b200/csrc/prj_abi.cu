@@ -452,6 +452,11 @@ int run_zsolve(prj_plan* pl, cudaStream_t st) {
         CK(prj::launch_zslab(pl, st), "z transform + Thomas (wavenumber on chip)");
         return PRJ_OK;
     }
+    if (prj::zline_cluster_selected(pl)) {
+        StageTimer tm(pl, prj::kStZSolve, st);
+        CK(prj::launch_zline_cluster(pl, st), "z transform + Thomas (cluster per wavenumber)");
+        return PRJ_OK;
+    }
     if (pl->zmode == 3) {
         StageTimer tm(pl, prj::kStZSolve, st);
         const cudaError_t e = prj::launch_zline(pl, st);
@@ -1162,7 +1167,7 @@ bool x_pass_active(const prj_plan* pl) { return pl->use_pass && pl->fx64.even &&
 int prj_plan_schedule(const prj_plan* plan, int mode, int* launches) {
     if (!plan || !launches) return fail(PRJ_ERR_ARG, "NULL argument");
     if (mode == PRJ_MODE_FP64) {
-        const bool one_z = prj::zslab_selected(plan) || !split_z(plan) || (plan->zmode == 3 && prj::zline_supported(plan));
+        const bool one_z = prj::zslab_selected(plan) || prj::zline_cluster_selected(plan) || !split_z(plan) || (plan->zmode == 3 && prj::zline_supported(plan));
         *launches = one_z ? 4 : 6;
     } else {
         // forward x, z transforms of the FP64 and FP32 rows, one Thomas launch, inverse z of both,

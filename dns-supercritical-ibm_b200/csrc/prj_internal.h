@@ -178,6 +178,10 @@ cudaError_t launch_zline(const prj_plan* pl, cudaStream_t st);
 // the plan's z tuning is the default and the wavenumber fits; else cudaErrorNotSupported
 cudaError_t launch_zslab(const prj_plan* pl, cudaStream_t st);
 bool zslab_selected(const prj_plan* pl);  // launch_zslab would run
+// the same as launch_zline with a cluster of CTAs per wavenumber (prj_zline.cu), or by it, where the
+// plan's z tuning is the default and its rule says so
+cudaError_t launch_zline_cluster(const prj_plan* pl, cudaStream_t st);
+bool zline_cluster_selected(const prj_plan* pl);  // launch_zline_cluster would run
 bool zline_supported(const prj_plan* pl);  // launch_zline would run (not fall back)
 
 // x transforms with the in-place DIF FFT (prj_xfft.cu); used when pl->xd.ok

@@ -37,6 +37,33 @@ cudaError_t launch_zline_pl(const ZLineArgs& a, const CUtensorMap& tm, size_t sm
     return cudaGetLastError();
 }
 
+// a cluster of a.C CTAs per wavenumber (two stages)
+template <class PL>
+__global__ void __launch_bounds__(zl_threads(PL::n, zl_lpt(PL::n)), zl_minb(zl_threads(PL::n, zl_lpt(PL::n))))
+    k_zline_cluster(const __grid_constant__ ZLineArgs a, const __grid_constant__ CUtensorMap tmap) {
+    extern __shared__ __align__(128) unsigned char zsm[];
+    zline_tile<PL, 2, zl_lpt(PL::n), zl_threads(PL::n, zl_lpt(PL::n)), 2, true>(a, &tmap, blockIdx.x / a.C, zsm);
+}
+
+template <class PL>
+cudaError_t launch_zline_cluster_pl(const ZLineArgs& a, const CUtensorMap& tm, size_t smem, cudaStream_t st) {
+    cudaError_t e =
+        cudaFuncSetAttribute(k_zline_cluster<PL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)(a.nh * a.C));
+    cfg.blockDim = dim3((unsigned)zl_threads(PL::n, zl_lpt(PL::n)));
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = (unsigned)a.C;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k_zline_cluster<PL>, a, tm);
+}
+
 template <class PL>
 cudaError_t launch_zline_ns(const ZLineArgs& a, const CUtensorMap& tm, int ns, size_t smem, cudaStream_t st) {
     constexpr int L = zl_lpt(PL::n);
@@ -108,19 +135,74 @@ bool zline_tmap(void* tmap128, const double2* X, int n, int nh, int ny, int yb) 
     return tmap_encode_f64(tmap128, X, 4, dims, strides, box);
 }
 
+// CTAs per wavenumber C and planes per chunk of the cluster form; C = 0 where it does not apply.
+// The most CTAs (up to 8) that are all resident at once: a second wave would double the chain.
+// C = 1 (k_zline) where there is a wavenumber per SM at least.  Measured (z solve, us, by cluster
+// / one CTA / three kernels): 58 / 74 / 83 at 256 x 128 x 128 (C = 3), 150 / 169 / 210 at
+// 384 x 192 x 192 (C = 2), 65 / 89 / 96 at 384 x 138 x 96, 50 / 56 / 58 at 192 x 42 x 384; - / 308 /
+// 398 at 512 x 256 x 256; but 132 / 198 / 92 at 64 x 130 x 512 and 107 / 222 / 60 at 64 x 53 x 768,
+// whose few wavenumbers have long rows (nz above 384 is left to the three kernels).
+static void zline_cluster_shape(const prj_plan* pl, int* C_out, int* yb_out) {
+    *C_out = *yb_out = 0;
+    const Geometry& g = pl->g;
+    // a z kernel, row count, ring, chunk or stage count chosen by the plan's tuning stands
+    if (pl->zmode != pl->zmode_default || (pl->zmode != 0 && pl->zmode != 3) || pl->zfft_rows != 0 ||
+        pl->thomas_async != -1 || pl->z_stages != 0 || pl->z_planes != 0)
+        return;
+    if (pl->sms <= 0 || !zline_supported(pl)) return;
+    const int nt = zl_threads(g.nz, zl_lpt(g.nz));
+    for (int C = g.nz <= 384 ? 8 : 1; C >= 2; C--) {
+        const int per_sm = (g.nxh * C + pl->sms - 1) / pl->sms;
+        if (per_sm > zl_minb(nt)) continue;
+        const size_t most = (size_t)228 * 1024 / per_sm - 1024;
+        int yb = 8;
+        while (yb > 1 && zline_cluster_smem(g.nz, g.mzp, yb, 2) > std::min(most, (size_t)220 * 1024)) yb--;
+        if (yb < 2 || yb * C > g.ny) continue;
+        *C_out = C;
+        *yb_out = yb;
+        return;
+    }
+    if (g.nxh >= pl->sms) *C_out = 1;
+}
+
+bool zline_cluster_selected(const prj_plan* pl) {
+    int C, yb;
+    zline_cluster_shape(pl, &C, &yb);
+    return C > 0;
+}
+
+cudaError_t launch_zline_cluster(const prj_plan* pl, cudaStream_t st) {
+    const Geometry& g = pl->g;
+    ZLineArgs a = zline_args(pl);
+    zline_cluster_shape(pl, &a.C, &a.yb);
+    if (a.C == 1) return launch_zline(pl, st);
+    CUtensorMap tm{};
+    if (a.C < 2 || !zline_tmap(&tm, pl->spec, g.nz, g.nxh, g.ny, a.yb)) return cudaErrorInvalidValue;
+    const size_t smem = zline_cluster_smem(g.nz, g.mzp, a.yb, 2);
+#define PRJ_ZL_CASE(N, ...)                                                  \
+    if (g.nz == N && same_radices<PassList<__VA_ARGS__>>(pl->zd.f))          \
+        return launch_zline_cluster_pl<PassList<__VA_ARGS__>>(a, tm, smem, st);
+    PRJ_PASS_ALL(PRJ_ZL_CASE)
+#undef PRJ_ZL_CASE
+    return cudaErrorInvalidValue;
+}
+
 // cudaErrorNotSupported when nz has no pass plan (the caller runs the split kernels)
 cudaError_t launch_zline(const prj_plan* pl, cudaStream_t st) {
     if (!pl->use_pass || !pl->zd.ok || !pl->kz_of_slot || !pl->t.pivc || !pl->spec) return cudaErrorNotSupported;
     const Geometry& g = pl->g;
     ZLineArgs a = zline_args(pl);
-    // planes per stage and stage count: the plan's z_planes / z_stages tuning, else 4 x 2;
-    // the planes per stage shrink until the ring fits 72 KB (three CTAs per SM).  Measured
-    // at 768x384x384 and not kept: deeper rings at fewer CTAs per SM, and one line per
-    // thread (twice the threads, spilling at the register budget of three CTAs per SM).
-    int yb = pl->z_planes > 0 ? pl->z_planes : 4, ns = pl->z_stages > 0 ? pl->z_stages : 2;
-    const size_t cap = (size_t)72 * 1024;
+    // planes per stage and stage count: the plan's z_planes / z_stages tuning, else two stages
+    // of up to 16 planes, as many as fit beside the CTAs that an SM is to hold (the wavenumbers
+    // per SM, as far as registers allow).  A chunk's barriers and waits are shared
+    // by its planes: 280 -> 256 us at 768 x 177 x 192 with 8 planes against 4; nz = 384 keeps
+    // 4.  Measured at 768x384x384 and not kept: deeper rings at fewer CTAs per SM, and one
+    // line per thread (twice the threads, spilling at the register budget of three CTAs).
+    int yb = pl->z_planes > 0 ? pl->z_planes : 16, ns = pl->z_stages > 0 ? pl->z_stages : 2;
+    const int sms = pl->sms > 0 ? pl->sms : 148;
+    const int per_sm = std::min(zl_minb(zl_threads(g.nz, zl_lpt(g.nz))), (g.nxh + sms - 1) / sms);
+    const size_t cap = std::min((size_t)228 * 1024 / per_sm - 1024, (size_t)200 * 1024);
     if (ns < 2 || ns > 4) ns = 2;
-    if (yb < 1) yb = 1;
     if (yb > g.ny) yb = g.ny;
     while (yb > 1 && zline_smem(g.nz, g.mzp, yb, ns) > cap) yb--;
     const size_t smem = zline_smem(g.nz, g.mzp, yb, ns);

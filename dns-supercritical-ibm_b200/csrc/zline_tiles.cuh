@@ -19,11 +19,13 @@
 // (poisson_solver_multigpu.f90:401-419, round-to-nearest intrinsics) are those of
 // k_zfft_pass and k_thomas, so the result is bitwise that of the split kernels.
 // Every mbarrier wait is bounded (a clock budget).  k_zline
-// (prj_zline.cu) runs one wavenumber per CTA; the persistent batch kernel
+// (prj_zline.cu) runs one wavenumber per CTA, k_zline_cluster one per cluster of CTAs that
+// take its chunks in turn; the persistent batch kernel
 // (prj_batchk.cu) runs (case, wavenumber) tiles from its work queue.
 #pragma once
 #include <cuda.h>
 
+#include "cluster_util.cuh"
 #include "cp_async.cuh"
 #include "div_rn.cuh"
 #include "fft_pass.cuh"
@@ -37,6 +39,7 @@ namespace prj {
 struct ZLineArgs {
     int ny, nh, mzp;
     int yb;               // planes per stage
+    int C;                // CTAs per wavenumber (cluster form)
     const double2* tw;    // z pass-plan twiddles
     const double* bands;  // a, b, c, a00, b00, c00
     const double* piv;    // D[y][kx][kzs]
@@ -46,11 +49,11 @@ struct ZLineArgs {
     int* err;             // raised (5) when a bounded mbarrier wait gives up
 };
 
-// lines per thread (default) and threads per CTA of a length-n plan; resident CTAs per
-// SM asked of the register allocator
-__host__ __device__ constexpr int zl_lpt(int n) { return n <= 128 ? 1 : n <= 512 ? 2 : n <= 1024 ? 4 : 8; }
-__host__ __device__ constexpr int zl_threads(int n, int lpt) { return n / lpt < 32 ? 32 : n / lpt; }
-__host__ __device__ constexpr int zl_minb(int nt) { return nt <= 64 ? 8 : nt <= 128 ? 5 : nt <= 384 ? 3 : 2; }
+// lines per thread and threads per CTA of a length-n plan (at least 128: the transforms of a
+// chunk's rows use them all); resident CTAs per SM asked of the register allocator
+__host__ __device__ constexpr int zl_lpt(int n) { return n <= 256 ? 1 : n <= 512 ? 2 : n <= 1024 ? 4 : 8; }
+__host__ __device__ constexpr int zl_threads(int n, int lpt) { return n / lpt < 128 ? 128 : n / lpt; }
+__host__ __device__ constexpr int zl_minb(int nt) { return nt <= 128 ? 5 : nt <= 384 ? 3 : 2; }
 
 // Pivot rows in shared memory: rows of mzs = mzp rounded up to 16 doubles; the 16-byte
 // piece j (kzs 2j, 2j+1) sits at piece zl_piece(j), which permutes the pieces of each
@@ -93,10 +96,16 @@ __host__ __device__ inline size_t zl_slot_bytes(int n, int yb) { return ((size_t
 // n; slots past n idle in the Thomas phase), NS stages of a.yb planes in `zsm`
 // (zline_smem bytes).  Each stage's rows arrive by one tensor-map copy (`tmap`:
 // zline_tmap's 4-D view of the spectrum) issued by thread 0 and completed on an mbarrier;
-// the pivot rows are cp.async copies (their pieces are permuted).  Every mbarrier wait is
-// bounded; UP planes of the forward sweep are unrolled: on a timeout the tile raises *a.err, waits (bounded) for its copies in flight
-// and returns.
-template <class PL, int NS, int LPT, int NT, int UP = 2>
+// the pivot rows are cp.async copies (their pieces are permuted).  UP planes of the forward
+// sweep are unrolled.  Every mbarrier wait is bounded: on a timeout the tile raises *a.err,
+// waits (bounded) for its copies in flight and returns.
+//
+// CL: the CTAs of a cluster of a.C share the wavenumber, CTA c taking the chunks c, c + C, ...
+// of both phases.  The sweeps stay one chain: d' of a chunk's last plane (x of its first on the
+// way down) goes to the next chunk's CTA by st.async into its carry row, completed on its
+// mbarrier; copies, transforms and the pivots' reciprocals (rbuf) of C chunks run meanwhile.
+// One carry row per direction is enough: the next carry depends on this CTA's own.
+template <class PL, int NS, int LPT, int NT, int UP = 2, bool CL = false>
 __device__ __forceinline__ void zline_tile(const ZLineArgs& a, const void* tmap, int kx, unsigned char* zsm) {
     constexpr int n = PL::n;
     static_assert(NT * LPT >= n, "every line has a thread");
@@ -109,13 +118,26 @@ __device__ __forceinline__ void zline_tile(const ZLineArgs& a, const void* tmap,
     unsigned char* rslots = base + 128;
     double* dring = reinterpret_cast<double*>(rslots + NS * slot_bytes);
     double* aring = dring + (size_t)NS * yb * mzs;  // a and a00 of each stage's planes
+    double* rbuf = aring + (size_t)NS * yb * 2;     // CL: reciprocals of the current chunk's pivots
+    double2* carry = reinterpret_cast<double2*>(rbuf + (size_t)yb * mzs);  // CL: up (n), down (n)
+    const int C = CL ? a.C : 1, rank = CL ? (int)cluster_rank() : 0;
+    const int nmine = (nch - rank + C - 1) / C;  // chunks rank, rank + C, ...
+    constexpr uint32_t carry_bytes = n * sizeof(double2);
+    // carries to come on the way up and down (every own chunk but the chain's first)
+    int left[2] = {nmine - (rank == 0 ? 1 : 0), nmine - ((nch - 1) % C == rank ? 1 : 0)};
     auto stage = [&](int s) { return reinterpret_cast<double2*>(rslots + s * slot_bytes); };
     if (tid == 0) {
 #pragma unroll
         for (int s = 0; s < NS; s++) mbar_init(&bars[s], 1);
+        if constexpr (CL)
+            for (int d = 0; d < 2; d++) mbar_init(&bars[NS + d], 1);
         mbar_fence_init();
+        if constexpr (CL)
+            for (int d = 0; d < 2; d++)
+                if (left[d] > 0) mbar_arrive_expect_tx(&bars[NS + d], carry_bytes);
     }
     __syncthreads();
+    if constexpr (CL) cluster_arrive();
     uint32_t phase = 0;    // bit s: parity of stage s's next completion
     uint32_t pending = 0;  // bit s: stage s has a copy in flight (the same in every thread)
 
@@ -132,13 +154,13 @@ __device__ __forceinline__ void zline_tile(const ZLineArgs& a, const void* tmap,
         is00[q] = (kx == 0 && kz == 0);
     }
 
-    // chunk c (planes c yb ..) into stage s with the rows of table tab (pivots on the way
+    // own chunk i, c = rank + i C (planes c yb ..), into stage s with the rows of table tab (pivots on the way
     // up, back-substitution factors on the way down): the rows by one tensor-map copy (a
     // box of yb planes, those past ny zero-filled), the pivots by every thread's cp.async
     // share; one cp.async group per call
-    auto issue = [&](int c, int s, const double* tab) {
-        if (c >= 0 && c < nch) {
-            const int y0 = c * yb, nr = min(yb, ny - y0);
+    auto issue = [&](int i, int s, const double* tab) {
+        if (i >= 0 && i < nmine) {
+            const int y0 = (rank + i * C) * yb, nr = min(yb, ny - y0);
             if (tid == 0) {
                 fence_proxy_async_shared();  // the stage's earlier reads before the copy's writes
                 mbar_arrive_expect_tx(&bars[s], (uint32_t)(18 * n * yb));
@@ -167,6 +189,25 @@ __device__ __forceinline__ void zline_tile(const ZLineArgs& a, const void* tmap,
         pending &= ~(1u << s);
         return !__syncthreads_or(!ok);
     };
+    // the carry of direction d (0 up, 1 down) into prev; false in every thread on a timeout
+    double2 prev[LPT];
+    uint32_t cphase[2] = {0, 0};
+    auto take = [&](int d) -> bool {
+        const bool ok = mbar_wait_cluster(&bars[NS + d], cphase[d]);
+        cphase[d] ^= 1u;
+        if (__syncthreads_or(!ok)) return false;
+#pragma unroll
+        for (int q = 0; q < LPT; q++) prev[q] = carry[d * n + at[q]];
+        left[d]--;
+        if (tid == 0 && left[d] > 0) mbar_arrive_expect_tx(&bars[NS + d], carry_bytes);
+        return true;
+    };
+    auto hand_on = [&](int d, int to) {
+        const uint32_t row = cluster_map(carry + d * n, (uint32_t)to), bar = cluster_map(&bars[NS + d], (uint32_t)to);
+#pragma unroll
+        for (int q = 0; q < LPT; q++)
+            if (slot[q] < n) st_async(row + (uint32_t)slot[q] * 16u, prev[q], bar);
+    };
     auto bail = [&]() {
         if (tid == 0) {
             atomicExch(a.err, 5);
@@ -179,18 +220,22 @@ __device__ __forceinline__ void zline_tile(const ZLineArgs& a, const void* tmap,
         if (tid == 0)
 #pragma unroll
             for (int s = 0; s < NS; s++) mbar_inval(&bars[s]);
+        if constexpr (CL) {  // no CTA leaves while a neighbour can still write to it
+            cluster_arrive();
+            cluster_wait();
+        }
     };
 
-    double2 prev[LPT];
 #pragma unroll
     for (int q = 0; q < LPT; q++) prev[q] = make_double2(0.0, 0.0);
 
     // ------------------------------------------------------------ forward phase
 #pragma unroll
-    for (int c = 0; c < NS - 1; c++) issue(c, c, a.piv);
-    for (int c = 0; c < nch; c++) {
-        issue(c + NS - 1, (c + NS - 1) % NS, a.piv);  // that stage was last read in iteration c - 1
-        const int s = c % NS, y0 = c * yb, nr = min(yb, ny - y0);
+    for (int i = 0; i < NS - 1; i++) issue(i, i, a.piv);
+    if constexpr (CL) cluster_wait();  // every CTA's mbarriers are set up
+    for (int i = 0; i < nmine; i++) {
+        issue(i + NS - 1, (i + NS - 1) % NS, a.piv);  // that stage was last read in iteration i - 1
+        const int s = i % NS, c = rank + i * C, y0 = c * yb, nr = min(yb, ny - y0);
         if (!acquire(s)) {
             bail();
             return;
@@ -198,7 +243,15 @@ __device__ __forceinline__ void zline_tile(const ZLineArgs& a, const void* tmap,
         double2* buf = stage(s);
         const double* dbuf = dring + (size_t)s * yb * mzs;
         const double* abuf = aring + (size_t)2 * s * yb;
+        if constexpr (CL)  // (pad entries too)
+            for (int k = tid; k < nr * mzs; k += NT) rbuf[k] = __drcp_rn(dbuf[k]);
         dif_passes_shared<-1, PL, 0, PL::P>(buf, nr, n, a.tw);  // barrier after every pass
+        if constexpr (CL) {
+            if (c > 0 && !take(0)) {
+                bail();
+                return;
+            }
+        }
         // plane by plane (lines past n run along on line 0's values and store nothing); a
         // quotient that may differ is noticed at the end of the chunk, whose inputs the stage
         // still holds
@@ -214,7 +267,7 @@ __device__ __forceinline__ void zline_tile(const ZLineArgs& a, const void* tmap,
             for (int q = 0; q < LPT; q++) {
                 v[q][0] = buf[sidx<true>(r * n + at[q])];
                 D[q][0] = dbuf[(size_t)r * mzs + kzs[q]];
-                rD[q][0] = __drcp_rn(D[q][0]);  // off the recurrence's chain
+                rD[q][0] = CL ? rbuf[(size_t)r * mzs + kzs[q]] : __drcp_rn(D[q][0]);  // off the chain
                 av[q][0] = y0 + r > 0 ? abuf[(is00[q] ? yb : 0) + r] : 0.0;
             }
             sweep_up<1, LPT>(v, D, rD, av, 1, prev, outside);
@@ -236,6 +289,8 @@ __device__ __forceinline__ void zline_tile(const ZLineArgs& a, const void* tmap,
                 }
             }
         }
+        if constexpr (CL)
+            if (c + 1 < nch) hand_on(0, (rank + 1) % C);
         __syncthreads();
     }
     cp_async_wait<0>();
@@ -246,19 +301,24 @@ __device__ __forceinline__ void zline_tile(const ZLineArgs& a, const void* tmap,
     __syncthreads();
 
     // ----------------------------------------------------------- backward phase
-    // j-th chunk from the top (chunk nch-1-j) uses stage (nch + j) % NS, continuing the
-    // forward phase's rotation
+    // own chunk nmine-1-j uses stage (nmine + j) % NS, continuing the forward phase's rotation
 #pragma unroll
-    for (int j = 0; j < NS - 1; j++) issue(nch - 1 - j, (nch + j) % NS, a.pivc);
-    for (int j = 0; j < nch; j++) {
-        issue(nch - 1 - (j + NS - 1), (nch + j + NS - 1) % NS, a.pivc);
-        const int s = (nch + j) % NS, c = nch - 1 - j, y0 = c * yb, nr = min(yb, ny - y0);
+    for (int j = 0; j < NS - 1; j++) issue(nmine - 1 - j, (nmine + j) % NS, a.pivc);
+    for (int j = 0; j < nmine; j++) {
+        issue(nmine - 1 - (j + NS - 1), (nmine + j + NS - 1) % NS, a.pivc);
+        const int s = (nmine + j) % NS, c = rank + (nmine - 1 - j) * C, y0 = c * yb, nr = min(yb, ny - y0);
         if (!acquire(s)) {
             bail();
             return;
         }
         double2* buf = stage(s);
         const double* dbuf = dring + (size_t)s * yb * mzs;
+        if constexpr (CL) {
+            if (c < nch - 1 && !take(1)) {
+                bail();
+                return;
+            }
+        }
         for (int r = nr - 1; r >= 0; r--) {
             const int y = y0 + r;
 #pragma unroll
@@ -277,6 +337,8 @@ __device__ __forceinline__ void zline_tile(const ZLineArgs& a, const void* tmap,
                 }
             }
         }
+        if constexpr (CL)
+            if (c > 0) hand_on(1, (rank + C - 1) % C);
         __syncthreads();
         dit_passes_shared<+1, PL, PL::P - 1, 0>(buf, nr, n, a.tw);
         dit_last_pass<+1, PL>(buf, nr, n, a.tw, [&](int r, int e, double2 v) {
@@ -298,6 +360,11 @@ ZLineArgs zline_args(const prj_plan* pl);
 // shared memory of a tile (alignment slack, mbarriers, row stages, pivot ring, a and a00)
 inline size_t zline_smem(int n, int mzp, int yb, int ns) {
     return 256 + (size_t)ns * zl_slot_bytes(n, yb) + (size_t)ns * yb * (zl_mzs(mzp) + 2) * sizeof(double);
+}
+
+// the same for a CTA of the cluster form (reciprocals and two carry rows more)
+inline size_t zline_cluster_smem(int n, int mzp, int yb, int ns) {
+    return zline_smem(n, mzp, yb, ns) + (size_t)yb * zl_mzs(mzp) * sizeof(double) + (size_t)2 * n * sizeof(double2);
 }
 
 // the 4-D tensor map of the row copies over the spectrum X (n-point z rows,
