@@ -10,6 +10,7 @@
 
 #include <vector>
 
+#include "chain.cuh"
 #include "fft_device.cuh"
 #include "fft_dif.cuh"
 
@@ -138,6 +139,9 @@ struct prj_plan {
 };
 
 namespace prj {
+
+// the plan's kernels are launched with launch_chained's attribute
+inline bool chained(const prj_plan* pl) { return (long long)pl->g.nx * pl->g.nz * pl->g.ny <= kChainPoints; }
 
 // Kernel launchers (prj_kernels.cu).  All are asynchronous on `st`.
 enum class FwdSource { Pressure, Divergence, Residual };

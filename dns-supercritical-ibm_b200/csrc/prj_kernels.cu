@@ -17,6 +17,7 @@
 // FMAs; only the pivots (not poi_C) are tabulated.
 #include <cstdio>
 
+#include "chain.cuh"
 #include "prj_internal.h"
 
 namespace prj {
@@ -335,6 +336,8 @@ struct CorrArgs {
 // y slices -1 and ny (and V at k = 0) take the wall values (:1234-1244).
 __global__ void __launch_bounds__(128) k_correct(const CorrArgs a) {
     // one block per halo'd x-row (jh, kh): no index division, coalesced along x
+    chain_trigger();
+    chain_wait();
     const int nx = a.nx, nz = a.nz, ny = a.ny;
     const int jh = blockIdx.y;
     const int k = (int)blockIdx.x + a.kh0 - 1;
@@ -521,8 +524,7 @@ cudaError_t launch_correction(const prj_plan* pl, const double* P, const double*
     for (int i = 0; i < 6; i++) a.wall[i] = sc.wall[i];
     if (kh.y1 <= kh.y0) return cudaSuccess;
     const dim3 grid((unsigned)(kh.y1 - kh.y0), (unsigned)(g.nz + 2));
-    k_correct<<<grid, 128, 0, st>>>(a);
-    return cudaGetLastError();
+    return launch_chained(chained(pl), k_correct, grid, 128, 0, st, 1, a);
 }
 
 cudaError_t launch_stats(const prj_plan* pl, const double* U, const double* V, const double* W, const double* P,

@@ -10,6 +10,7 @@
 // needs one row buffer per x-row, half of an out-of-place transform, so more
 // CTAs fit on an SM.  Loads and stores of P and u_hat are one element per
 // thread along x (fully coalesced).
+#include "chain.cuh"
 #include "fft_dif.cuh"
 #include "fft_host.h"
 #include "fft_pass.cuh"
@@ -226,15 +227,25 @@ __global__ void __launch_bounds__(256, PRJ_FFT_MINB) k_bwd_xd(const XArgs a) {
 // CTA (the last CTA may hold fewer).
 
 // k_fwd_xp / k_bwd_xp: one CTA per tile of the pass-plan x transforms (xfft_tiles.cuh)
-template <int SRC, class PL>
+// CH: launched with launch_chained (its own instance: the wait's memory clobber costs the
+// pressure loads their read-only path, 117 -> 187 us at 512 x 256 x 256)
+template <int SRC, class PL, bool CH>
 __global__ void __launch_bounds__(x_threads(PL::n), x_minb(PL::n)) k_fwd_xp(const XArgs a) {
     extern __shared__ __align__(16) unsigned char sm[];
+    if constexpr (CH) {
+        chain_trigger();
+        chain_wait();
+    }
     fwd_xp_tile<SRC, PL>(a, sm, blockIdx.x, blockIdx.y);
 }
 
-template <class PL>
+template <class PL, bool CH>
 __global__ void __launch_bounds__(x_threads(PL::n), x_minb(PL::n)) k_bwd_xp(const XArgs a) {
     extern __shared__ __align__(16) unsigned char sm[];
+    if constexpr (CH) {
+        chain_trigger();
+        chain_wait();
+    }
     bwd_xp_tile<PL>(a, sm, blockIdx.x, blockIdx.y, gridDim.x);
 }
 
@@ -310,30 +321,32 @@ size_t pass_smem_bytes(const XArgs& a) {
     return (size_t)padded_len(a.tz * pass_row_stride(a.m), true) * sizeof(double2);
 }
 
-template <class PL>
-cudaError_t launch_fwd_xp_pl(const XArgs& a, FwdSource src, const dim3& grid, cudaStream_t st) {
+template <class PL, int SRC, bool CH>
+cudaError_t launch_fwd_xp_src(const XArgs& a, const dim3& grid, cudaStream_t st) {
     const size_t smem = pass_smem_bytes(a);
-    cudaError_t e;
-    if (src == FwdSource::Pressure) {
-        if ((e = allow_smem(k_fwd_xp<0, PL>, smem)) != cudaSuccess) return e;
-        k_fwd_xp<0, PL><<<grid, x_threads(PL::n), smem, st>>>(a);
-    } else if (src == FwdSource::Residual) {
-        if ((e = allow_smem(k_fwd_xp<3, PL>, smem)) != cudaSuccess) return e;
-        k_fwd_xp<3, PL><<<grid, x_threads(PL::n), smem, st>>>(a);
-    } else {
-        if ((e = allow_smem(k_fwd_xp<1, PL>, smem)) != cudaSuccess) return e;
-        k_fwd_xp<1, PL><<<grid, x_threads(PL::n), smem, st>>>(a);
-    }
-    return cudaGetLastError();
+    const cudaError_t e = allow_smem(k_fwd_xp<SRC, PL, CH>, smem);
+    return e != cudaSuccess ? e : launch_chained(CH, k_fwd_xp<SRC, PL, CH>, grid, x_threads(PL::n), smem, st, 1, a);
+}
+
+// the residual source belongs to the mixed-precision path, which is not chained
+template <class PL>
+cudaError_t launch_fwd_xp_pl(const XArgs& a, FwdSource src, const dim3& grid, bool chained, cudaStream_t st) {
+    if (src == FwdSource::Residual) return launch_fwd_xp_src<PL, 3, false>(a, grid, st);
+    if (src == FwdSource::Pressure)
+        return chained ? launch_fwd_xp_src<PL, 0, true>(a, grid, st) : launch_fwd_xp_src<PL, 0, false>(a, grid, st);
+    return chained ? launch_fwd_xp_src<PL, 1, true>(a, grid, st) : launch_fwd_xp_src<PL, 1, false>(a, grid, st);
+}
+
+template <class PL, bool CH>
+cudaError_t launch_bwd_xp_ch(const XArgs& a, const dim3& grid, cudaStream_t st) {
+    const size_t smem = pass_smem_bytes(a);
+    const cudaError_t e = allow_smem(k_bwd_xp<PL, CH>, smem);
+    return e != cudaSuccess ? e : launch_chained(CH, k_bwd_xp<PL, CH>, grid, x_threads(PL::n), smem, st, 1, a);
 }
 
 template <class PL>
-cudaError_t launch_bwd_xp_pl(const XArgs& a, const dim3& grid, cudaStream_t st) {
-    const size_t smem = pass_smem_bytes(a);
-    cudaError_t e = allow_smem(k_bwd_xp<PL>, smem);
-    if (e != cudaSuccess) return e;
-    k_bwd_xp<PL><<<grid, x_threads(PL::n), smem, st>>>(a);
-    return cudaGetLastError();
+cudaError_t launch_bwd_xp_pl(const XArgs& a, const dim3& grid, bool chained, cudaStream_t st) {
+    return chained ? launch_bwd_xp_ch<PL, true>(a, grid, st) : launch_bwd_xp_ch<PL, false>(a, grid, st);
 }
 
 // x kernels for even nx: the half length's compile-time pass plan, or the runtime radices;
@@ -342,14 +355,15 @@ cudaError_t launch_xpass(const prj_plan* pl, bool fwd, FwdSource src, XArgs a, i
     a.tz = pl->tz_xp;
     if (!pl->use_pass || !a.even || !pl->xd.ok || pass_smem_bytes(a) > (size_t)200 * 1024) return cudaErrorNotSupported;
     const dim3 grid((pl->g.nz + a.tz - 1) / a.tz, ny_launch);
+    const bool ch = chained(pl);
 #define PRJ_X_CASE(N, ...)                                                                          \
     if (a.m == N && same_radices<PassList<__VA_ARGS__>>(pl->xd.f)) {                                \
         using PL = PassList<__VA_ARGS__>;                                                           \
-        return fwd ? launch_fwd_xp_pl<PL>(a, src, grid, st) : launch_bwd_xp_pl<PL>(a, grid, st);    \
+        return fwd ? launch_fwd_xp_pl<PL>(a, src, grid, ch, st) : launch_bwd_xp_pl<PL>(a, grid, ch, st); \
     }
     PRJ_PASS_ALL(PRJ_X_CASE)
 #undef PRJ_X_CASE
-    return fwd ? launch_fwd_xp_pl<RuntimePlan>(a, src, grid, st) : launch_bwd_xp_pl<RuntimePlan>(a, grid, st);
+    return fwd ? launch_fwd_xp_pl<RuntimePlan>(a, src, grid, ch, st) : launch_bwd_xp_pl<RuntimePlan>(a, grid, ch, st);
 }
 
 }  // namespace

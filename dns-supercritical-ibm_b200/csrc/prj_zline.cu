@@ -11,6 +11,7 @@
 // kernels.
 #include <cuda.h>
 
+#include "chain.cuh"
 #include "div_rn.cuh"
 #include "fft_pass.cuh"
 #include "prj_internal.h"
@@ -50,18 +51,8 @@ cudaError_t launch_zline_cluster_pl(const ZLineArgs& a, const CUtensorMap& tm, s
     cudaError_t e =
         cudaFuncSetAttribute(k_zline_cluster<PL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)(a.nh * a.C));
-    cfg.blockDim = dim3((unsigned)zl_threads(PL::n, zl_lpt(PL::n)));
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = (unsigned)a.C;
-    at.val.clusterDim.y = at.val.clusterDim.z = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_zline_cluster<PL>, a, tm);
+    return launch_chained(false, k_zline_cluster<PL>, dim3((unsigned)(a.nh * a.C)), zl_threads(PL::n, zl_lpt(PL::n)), smem, st,
+                          (unsigned)a.C, a, tm);
 }
 
 template <class PL>

@@ -26,6 +26,7 @@
 // incoming stores are the ones it has waited for.
 #include <cuda.h>
 
+#include "chain.cuh"
 #include "cluster_util.cuh"
 #include "cp_async.cuh"
 #include "div_rn.cuh"
@@ -119,6 +120,7 @@ template <class FFT, int NT, int LPT>
 __global__ void __launch_bounds__(NT, 512 / NT) k_zslab(const __grid_constant__ ZSlabArgs a,
                                                         const __grid_constant__ CUtensorMap tmap) {
     extern __shared__ __align__(128) unsigned char zsm[];
+    chain_trigger();
     const int tid = threadIdx.x, c = (int)cluster_rank(), C = (int)gridDim.x, kx = blockIdx.y;
     const int n = a.n, ny = a.ny, nh = a.nh, rs = a.rs, H = a.H, hp = a.hp;
     const int y0 = c * H, nr = min(H, ny - y0);  // at least one plane per CTA
@@ -135,20 +137,10 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_zslab(const __grid_constant__ 
         mbar_init(&bars[0], 1);
         mbar_init(&bars[1], 1);
         mbar_fence_init();
-        if (a.tma) {
-            mbar_arrive_expect_tx(&bars[0], (uint32_t)(slab_row_bytes(n) * a.H));
-            tma_load_4d(buf, &tmap, 0, 0, kx, y0, &bars[0]);
-        }
         // the first carry: d' from below, or (CTA 0) x from above
         if (C > 1) mbar_arrive_expect_tx(&bars[1], carry_bytes);
     }
     cluster_arrive();  // this CTA's mbarriers are set up (waited for before the first st_async)
-    if (!a.tma) {
-        for (int r = 0; r < nr; r++) {
-            const double2* src = a.X + ((size_t)(y0 + r) * nh + kx) * n;
-            for (int e = tid; e < n; e += NT) cp_async(buf + (size_t)r * rp + e + (e >> 3), src + e, 16);
-        }
-    }
     for (int i = tid; i < 4 * nr; i += NT) {  // a, a00, c, c00 of the planes
         const int k = i / nr, r = i - k * nr;
         cp_async(abuf + k * H + r, a.bands + (size_t)((k & 1) * 3 + (k >> 1) * 2) * ny + y0 + r, 8);
@@ -183,6 +175,20 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_zslab(const __grid_constant__ 
         const int sq = slot[q] < n ? slot[q] : 0;
         at[q] = sq + (sq >> 3);
         piv[q] = a.pair[sq] * hp;
+    }
+    // the rows, once the kernel that wrote them is done
+    chain_wait();
+    if (a.tma) {
+        if (tid == 0) {
+            mbar_arrive_expect_tx(&bars[0], (uint32_t)(slab_row_bytes(n) * a.H));
+            tma_load_4d(buf, &tmap, 0, 0, kx, y0, &bars[0]);
+        }
+    } else {
+        for (int r = 0; r < nr; r++) {
+            const double2* src = a.X + ((size_t)(y0 + r) * nh + kx) * n;
+            for (int e = tid; e < n; e += NT) cp_async(buf + (size_t)r * rp + e + (e >> 3), src + e, 16);
+        }
+        cp_async_commit();
     }
     cp_async_wait<0>();
     bool ok = true;
@@ -360,28 +366,18 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_zslab(const __grid_constant__ 
 }
 
 template <class FFT, int NT, int LPT>
-cudaError_t launch_slab(const ZSlabArgs& a, const CUtensorMap& tm, int C, size_t smem, cudaStream_t st) {
+cudaError_t launch_slab(const ZSlabArgs& a, const CUtensorMap& tm, int C, size_t smem, bool chained, cudaStream_t st) {
     auto kernel = k_zslab<FFT, NT, LPT>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)C, (unsigned)a.nh);
-    cfg.blockDim = dim3(NT);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = (unsigned)C;
-    at.val.clusterDim.y = at.val.clusterDim.z = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, a, tm);
+    return launch_chained(chained, kernel, dim3((unsigned)C, (unsigned)a.nh), NT, smem, st, (unsigned)C, a, tm);
 }
 
 template <class FFT, int N>
-cudaError_t launch_slab_n(const ZSlabArgs& a, const CUtensorMap& tm, int C, size_t smem, cudaStream_t st) {
+cudaError_t launch_slab_n(const ZSlabArgs& a, const CUtensorMap& tm, int C, size_t smem, bool chained,
+                          cudaStream_t st) {
     constexpr int NT = 256, LPT = (N + NT - 1) / NT;
-    return launch_slab<FFT, NT, LPT>(a, tm, C, smem, st);
+    return launch_slab<FFT, NT, LPT>(a, tm, C, smem, chained, st);
 }
 
 }  // namespace
@@ -430,14 +426,15 @@ cudaError_t launch_zslab(const prj_plan* pl, cudaStream_t st) {
     a.tma = zline_tmap(&tm, pl->spec, g.nz, g.nxh, g.ny, H) ? 1 : 0;
     const int C = (g.ny + H - 1) / H;
     const size_t smem = slab_smem(g.nz, H);
+    const bool ch = chained(pl);
 #define PRJ_SLAB_CASE(N, ...)                                                            \
     if (g.nz == N && same_radices<PassList<__VA_ARGS__>>(pl->zd.f))                      \
-        return launch_slab_n<PassFft<PassList<__VA_ARGS__>>, N>(a, tm, C, smem, st);
+        return launch_slab_n<PassFft<PassList<__VA_ARGS__>>, N>(a, tm, C, smem, ch, st);
     PRJ_PASS_ALL(PRJ_SLAB_CASE)
 #undef PRJ_SLAB_CASE
-    if (g.nz <= 256) return launch_slab<RuntimeFft, 256, 1>(a, tm, C, smem, st);
-    if (g.nz <= 512) return launch_slab<RuntimeFft, 256, 2>(a, tm, C, smem, st);
-    if (g.nz <= 1024) return launch_slab<RuntimeFft, 256, 4>(a, tm, C, smem, st);
+    if (g.nz <= 256) return launch_slab<RuntimeFft, 256, 1>(a, tm, C, smem, ch, st);
+    if (g.nz <= 512) return launch_slab<RuntimeFft, 256, 2>(a, tm, C, smem, ch, st);
+    if (g.nz <= 1024) return launch_slab<RuntimeFft, 256, 4>(a, tm, C, smem, ch, st);
     return cudaErrorNotSupported;
 }
 
