@@ -678,8 +678,8 @@ int prj_plan_create(int nx, int nz, int ny, double dx, double dz, const double* 
         pl->sms = sms;
         pl->zmode = pl->zmode_default = z_mode(prj::smooth5(nz), sms > 0 && g.nxh >= 2 * sms);
     }
-    // pass-plan kernels wherever the length has a plan; the Thomas ring for the
-    // mixed-storage solve only (prj_tuning.thomas_ring changes it)
+    // pass-plan kernels wherever the length has a plan; the Thomas kernel by its default rule
+    // (prj_tuning.thomas_ring changes it)
     pl->use_pass = true;
     pl->thomas_async = -1;
     pl->kxs = g.nxh;

@@ -127,7 +127,7 @@ struct prj_plan {
     int sms = 0;                  // SMs of the plan's device
     bool use_pass = true;         // compile-time pass-plan FFT kernels where the length has one
     int thomas_async = -1;        // Thomas lines streamed through a cp.async shared-memory ring:
-                                  // -1 for the mixed storage only, 0 never, 1..4 always (ring shape)
+                                  // -1 and 0 never, 1..4 always (ring shape)
     int tz_xp = 1;                // rows per CTA of the pass-plan x kernels
     double* vd_pad = nullptr;     // inv_dy_p_pad (ny+1) of the variable-density step
     double* vd_ih = nullptr;      // 0.5 / rho (halo'd) of the variable-density step (scratch)

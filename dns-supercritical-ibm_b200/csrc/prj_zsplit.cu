@@ -326,14 +326,17 @@ cudaError_t launch_thomas_mixed(const prj_plan* pl, cudaStream_t st) {
     const ThomasArgs a32 = thomas_args(pl, pl->spec32, pl->kxs, rows32);
     const int nblk64 = pl->kxs * a64.tiles;
     const unsigned grid = (unsigned)(nblk64 + rows32 * a32.tiles);
-    // the mixed storage streams by default (measured 0.69 ms against 1.10 ms per solve at
-    // 768x384x384); thomas_ring 0 keeps the register-prefetch kernel
-    switch (pl->thomas_async) {
-    case 0: break;
+    // register prefetch by default: since its quotients run without branches it takes 0.44 ms per
+    // solve at 768x384x384 against 0.57 ms for the best ring (1.10 and 0.59 ms with them); below
+    // two CTAs per SM, where few loads are in flight, the ring of 8 planes by 2 stages (41 / 46 us
+    // per solve at 240x120x150, 74 / 90 at 64x324x80; 164 / 142 at 512x256x256)
+    const int ring = pl->thomas_async < 0 ? (grid < 2u * (unsigned)pl->sms ? 2 : 0) : pl->thomas_async;
+    switch (ring) {
+    case 1: return launch_thomas_mixed_async<4, 4>(a64, a32, nblk64, grid, st);
     case 2: return launch_thomas_mixed_async<8, 2>(a64, a32, nblk64, grid, st);
     case 3: return launch_thomas_mixed_async<2, 8>(a64, a32, nblk64, grid, st);
     case 4: return launch_thomas_mixed_async<8, 3>(a64, a32, nblk64, grid, st);
-    default: return launch_thomas_mixed_async<4, 4>(a64, a32, nblk64, grid, st);
+    default: break;
     }
     k_thomas_mixed<<<grid, kThomasTile, 0, st>>>(a64, a32, nblk64);
     return cudaGetLastError();

@@ -51,6 +51,32 @@ __device__ __forceinline__ void zfft_stage(const ZfftArgs& a, double2* S, int bx
     cp_async_commit();
 }
 
+// `tot` elements of whole rows, contiguous in X, to and from padded slots; 16 bytes per access
+// (FP32 rows two elements at a time: a pass-plan length is even, so every row is 16-byte aligned)
+__device__ __forceinline__ void load_rows(double2* zp, const double2* X, int tot) {
+#pragma unroll 4
+    for (int i = threadIdx.x; i < tot; i += blockDim.x) zp[sidx<true>(i)] = X[i];
+}
+__device__ __forceinline__ void load_rows(double2* zp, const float2* X, int tot) {
+    const float4* X4 = reinterpret_cast<const float4*>(X);
+#pragma unroll 4
+    for (int i = threadIdx.x; i < tot / 2; i += blockDim.x) {
+        const float4 v = X4[i];
+        zp[sidx<true>(2 * i)] = make_double2(v.x, v.y);
+        zp[sidx<true>(2 * i + 1)] = make_double2(v.z, v.w);
+    }
+}
+__device__ __forceinline__ void store_rows(double2* X, const double2* zp, int tot) {
+    for (int i = threadIdx.x; i < tot; i += blockDim.x) X[i] = zp[sidx<true>(i)];
+}
+__device__ __forceinline__ void store_rows(float2* X, const double2* zp, int tot) {
+    float4* X4 = reinterpret_cast<float4*>(X);
+    for (int i = threadIdx.x; i < tot / 2; i += blockDim.x) {
+        const double2 a = zp[sidx<true>(2 * i)], b = zp[sidx<true>(2 * i + 1)];
+        X4[i] = make_float4((float)a.x, (float)a.y, (float)b.x, (float)b.y);
+    }
+}
+
 // STAGED: the rows come from S, where zfft_stage put them, and after_load() is called
 // once S is no longer read
 template <int DIR, typename T, class PL, bool STAGE_INV = false, bool STAGED = false, class Hook = NoHook>
@@ -76,15 +102,14 @@ __device__ __forceinline__ void zfft_pass_tile(const ZfftArgs& a, double2* zp, i
         __syncthreads();
         after_load();
         dif_passes_shared<-1, PL, 1, PL::P>(zp, nr, n, tw);
-        for (int i = threadIdx.x; i < tot; i += blockDim.x) from_d2(X[i], zp[sidx<true>(i)]);
+        store_rows(X, zp, tot);
     } else {
         if (STAGE_INV) {
             // slot-order rows copied in whole (coalesced), every pass in shared memory
             if constexpr (STAGED) {
                 for (int i = threadIdx.x; i < tot; i += blockDim.x) zp[sidx<true>(i)] = S[i];
             } else {
-#pragma unroll 4
-                for (int i = threadIdx.x; i < tot; i += blockDim.x) zp[sidx<true>(i)] = to_d2(X[i]);
+                load_rows(zp, X, tot);
             }
             __syncthreads();
             after_load();

@@ -312,11 +312,15 @@ int prj_batch_destroy(prj_batch* batch);
  *               lengths with a prime factor above 5), 2 = its unpipelined form,
  *               3 = one kernel per x wavenumber on the compile-time pass plans (the
  *               three kernels where nz has no pass plan).  The default is 3 when
- *               nx/2+1 >= 2 x the SM count, else 0;
- *   z_planes    planes per chunk of the per-wavenumber z kernels (0 = default);
+ *               nx/2+1 >= 2 x the SM count, else 0 (1 for nz with a prime factor above 5).
+ *               With this and the next knobs at their defaults the plan picks by size:
+ *               a whole x wavenumber on chip, one kernel per x wavenumber by one CTA or a
+ *               cluster of them, or the three kernels (nz of any factors); the same bits;
+ *   z_planes    planes per chunk of the per-wavenumber z kernels, planes per CTA of the
+ *               on-chip one (0 = default);
  *   z_stages    stages of their copy rings (0 = default, else 2..4; 2..8 for mode 1);
- *   thomas_ring shared-memory ring of the split Thomas kernel: -1 = default (the
- *               mixed storage only), 0 = none, 1..4 = shapes 4x4, 8x2, 2x8, 8x3
+ *   thomas_ring shared-memory ring of the split Thomas kernel: -1 = default (none),
+ *               0 = none, 1..4 = shapes 4x4, 8x2, 2x8, 8x3
  *               (planes x stages) for both storages;
  *   mixed_iters refinement passes of PRJ_MODE_FP32_REFINE (default 1, 0..8);
  *   mixed_tau   x-wavenumber rows with |a_x| < mixed_tau max|b| keep FP64 storage in
