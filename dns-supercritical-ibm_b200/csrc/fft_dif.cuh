@@ -119,6 +119,22 @@ __device__ __noinline__ void stage_r(V* buf, int nrows, int rs, int nb, int mm, 
     }
 }
 
+// stage s of the plan, whatever its radix
+template <int DIR, bool DIT, bool PAD, typename V>
+__device__ __forceinline__ void stage_switch(V* buf, int nrows, int rs, const DifDev& f, int s, const V* __restrict__ tw) {
+    const int R = f.radix[s], nb = f.n / R, mm = f.span[s] / R;
+    const V* w = tw + f.twoff[s];
+    const FastDiv dnb = f.nbdiv[s], dmm = f.mmdiv[s];
+    switch (R) {
+#define PRJ_STAGE(R_) \
+    case R_: stage_r<DIR, DIT, PAD, R_>(buf, nrows, rs, nb, mm, dnb, dmm, w); break;
+        PRJ_STAGE(2) PRJ_STAGE(3) PRJ_STAGE(4) PRJ_STAGE(5) PRJ_STAGE(6) PRJ_STAGE(7) PRJ_STAGE(8)
+        PRJ_STAGE(9) PRJ_STAGE(10) PRJ_STAGE(11) PRJ_STAGE(13)
+#undef PRJ_STAGE
+    default: break;  // the host plans no other radix here (dif_supported)
+    }
+}
+
 // In-place transform of `nrows` rows of n elements (row r starts at element
 // r * rs; with PAD, element g of the buffer lives at slot g + g/8).  DIT = false:
 // decimation in frequency, natural order in, digit-reversed out.  DIT = true:
@@ -128,19 +144,58 @@ __device__ __noinline__ void stage_r(V* buf, int nrows, int rs, int nb, int mm, 
 template <int DIR, bool DIT, bool PAD, typename V>
 __device__ __forceinline__ void inplace_rows(V* buf, int nrows, int rs, const DifDev& f, const V* __restrict__ tw) {
     for (int t = 0; t < f.nst; t++) {
-        const int s = DIT ? f.nst - 1 - t : t;
-        const int R = f.radix[s], nb = f.n / R, mm = f.span[s] / R;
-        const V* w = tw + f.twoff[s];
-        const FastDiv dnb = f.nbdiv[s], dmm = f.mmdiv[s];
-        switch (R) {
-#define PRJ_STAGE(R_) \
-    case R_: stage_r<DIR, DIT, PAD, R_>(buf, nrows, rs, nb, mm, dnb, dmm, w); break;
-            PRJ_STAGE(2) PRJ_STAGE(3) PRJ_STAGE(4) PRJ_STAGE(5) PRJ_STAGE(6) PRJ_STAGE(7) PRJ_STAGE(8)
-            PRJ_STAGE(9) PRJ_STAGE(10) PRJ_STAGE(11) PRJ_STAGE(13)
-#undef PRJ_STAGE
-        default: break;  // the host plans no other radix here (dif_supported)
-        }
+        stage_switch<DIR, DIT, PAD>(buf, nrows, rs, f, DIT ? f.nst - 1 - t : t, tw);
         __syncthreads();
+    }
+}
+
+// rows of whole elements at a stride in memory, a sink of dit_rows_to
+__device__ __forceinline__ void put(double2* p, double2 v) { *p = v; }
+__device__ __forceinline__ void put(float2* p, double2 v) { *p = make_float2((float)v.x, (float)v.y); }
+template <typename T>
+struct RowStore {
+    T* p;
+    size_t stride;
+    __device__ __forceinline__ void operator()(int r, int e, double2 v) const { put(p + r * stride + e, v); }
+};
+
+// the last stage of a decimation in time (span n), its natural-order outputs to st(row, e, value)
+template <int DIR, int R, typename V, class St>
+__device__ __noinline__ void stage_out_r(const V* buf, int nrows, int rs, int mm, FastDiv dmm, const V* __restrict__ w,
+                                         St st) {
+    for (int idx = threadIdx.x; idx < mm * nrows; idx += blockDim.x) {
+        const int row = fdiv(idx, dmm), j = idx - row * mm;
+        V a[R];
+#pragma unroll
+        for (int q = 0; q < R; q++) a[q] = buf[sidx<true>(row * rs + j + q * mm)];
+        if (j) apply_twiddles<DIR, R>(a, w, j);
+        dft_r<DIR, R>(a);
+#pragma unroll
+        for (int q = 0; q < R; q++) st(row, j + q * mm, a[q]);
+    }
+}
+
+// inplace_rows with DIT = true and PAD, its result to st instead of shared memory (one round
+// trip and one barrier fewer).  No barrier at the end.
+template <int DIR, typename V, class St>
+__device__ __forceinline__ void dit_rows_to(V* buf, int nrows, int rs, const DifDev& f, const V* __restrict__ tw, St st) {
+    for (int s = f.nst - 1; s > 0; s--) {
+        stage_switch<DIR, true, true>(buf, nrows, rs, f, s, tw);
+        __syncthreads();
+    }
+    if (f.nst == 0) {  // n = 1
+        for (int r = threadIdx.x; r < nrows; r += blockDim.x) st(r, 0, buf[sidx<true>(r * rs)]);
+        return;
+    }
+    const int mm = f.span[0] / f.radix[0];
+    const FastDiv dmm = f.mmdiv[0];
+    switch (f.radix[0]) {
+#define PRJ_STAGE(R_) \
+    case R_: stage_out_r<DIR, R_>(buf, nrows, rs, mm, dmm, tw + f.twoff[0], st); break;
+        PRJ_STAGE(2) PRJ_STAGE(3) PRJ_STAGE(4) PRJ_STAGE(5) PRJ_STAGE(6) PRJ_STAGE(7) PRJ_STAGE(8)
+        PRJ_STAGE(9) PRJ_STAGE(10) PRJ_STAGE(11) PRJ_STAGE(13)
+#undef PRJ_STAGE
+    default: break;
     }
 }
 

@@ -103,7 +103,7 @@ constexpr int kBatchMinBlocks = PRJ_BATCH_MINB;
 template <class PL, bool FWD>
 __device__ __forceinline__ void run_x_tiles(const BatchCaseDev& c, const CUtensorMap* xmap, int t0, int count,
                                             unsigned char* sm, int* err) {
-    x_tiles_tma<PL, FWD, false>(c.x, xmap, c.ntz, c.xboxes, c.xbox_k, sm, c.soff, c.sbytes, t0, 1, t0 + count, err);
+    x_tiles_tma<PL, FWD>(c.x, xmap, c.ntz, c.xboxes, c.xbox_k, sm, c.soff, c.sbytes, t0, 1, t0 + count, err);
 }
 template <class PL>
 __device__ __noinline__ void run_x_fwd_tiles(const BatchCaseDev& c, const CUtensorMap* xmap, int t0, int count,

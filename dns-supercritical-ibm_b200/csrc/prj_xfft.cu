@@ -239,14 +239,14 @@ __global__ void __launch_bounds__(x_threads(PL::n), x_minb(PL::n)) k_fwd_xp(cons
     fwd_xp_tile<SRC, PL>(a, sm, blockIdx.x, blockIdx.y);
 }
 
-template <class PL, bool CH>
+template <class PL, bool CH, int EX>
 __global__ void __launch_bounds__(x_threads(PL::n), x_minb(PL::n)) k_bwd_xp(const XArgs a) {
     extern __shared__ __align__(16) unsigned char sm[];
     if constexpr (CH) {
         chain_trigger();
         chain_wait();
     }
-    bwd_xp_tile<PL>(a, sm, blockIdx.x, blockIdx.y, gridDim.x);
+    bwd_xp_tile<PL, EX>(a, sm, blockIdx.x, blockIdx.y, gridDim.x);
 }
 
 XArgs make_args(const prj_plan* pl) {
@@ -337,16 +337,19 @@ cudaError_t launch_fwd_xp_pl(const XArgs& a, FwdSource src, const dim3& grid, bo
     return chained ? launch_fwd_xp_src<PL, 1, true>(a, grid, st) : launch_fwd_xp_src<PL, 1, false>(a, grid, st);
 }
 
-template <class PL, bool CH>
-cudaError_t launch_bwd_xp_ch(const XArgs& a, const dim3& grid, cudaStream_t st) {
+template <class PL, bool CH, int EX>
+cudaError_t launch_bwd_xp_ex(const XArgs& a, const dim3& grid, cudaStream_t st) {
     const size_t smem = pass_smem_bytes(a);
-    const cudaError_t e = allow_smem(k_bwd_xp<PL, CH>, smem);
-    return e != cudaSuccess ? e : launch_chained(CH, k_bwd_xp<PL, CH>, grid, x_threads(PL::n), smem, st, 1, a);
+    const cudaError_t e = allow_smem(k_bwd_xp<PL, CH, EX>, smem);
+    return e != cudaSuccess ? e : launch_chained(CH, k_bwd_xp<PL, CH, EX>, grid, x_threads(PL::n), smem, st, 1, a);
 }
 
+// accumulation and partial sums belong to the mixed-precision path, which is not chained
 template <class PL>
 cudaError_t launch_bwd_xp_pl(const XArgs& a, const dim3& grid, bool chained, cudaStream_t st) {
-    return chained ? launch_bwd_xp_ch<PL, true>(a, grid, st) : launch_bwd_xp_ch<PL, false>(a, grid, st);
+    if (a.accum) return launch_bwd_xp_ex<PL, false, 2>(a, grid, st);
+    if (a.psum) return launch_bwd_xp_ex<PL, false, 1>(a, grid, st);
+    return chained ? launch_bwd_xp_ex<PL, true, 0>(a, grid, st) : launch_bwd_xp_ex<PL, false, 0>(a, grid, st);
 }
 
 // x kernels for even nx: the half length's compile-time pass plan, or the runtime radices;

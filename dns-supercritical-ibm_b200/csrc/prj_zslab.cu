@@ -74,9 +74,7 @@ struct RuntimeFft {
     }
     template <class St>
     static __device__ __forceinline__ void inverse(double2* buf, int nr, int rs, const ZSlabArgs& a, St st) {
-        inplace_rows<+1, true, true>(buf, nr, rs, a.f, a.tw);
-        for (int r = 0; r < nr; r++)
-            for (int e = threadIdx.x; e < a.n; e += blockDim.x) st(r, e, buf[sidx<true>(r * rs + e)]);
+        dit_rows_to<+1>(buf, nr, rs, a.f, a.tw, st);
     }
 };
 
@@ -356,7 +354,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_zslab(const __grid_constant__ 
                 if (slot[q] < n) st_async(dn + (uint32_t)slot[q] * 16u, prev[q], dnbar);
         }
         __syncthreads();
-        FFT::inverse(buf, nr, rs, a, [&](int r, int e, double2 v) { a.X[((size_t)(y0 + r) * nh + kx) * n + e] = v; });
+        FFT::inverse(buf, nr, rs, a, RowStore<double2>{a.X + ((size_t)y0 * nh + kx) * n, (size_t)nh * n});
     }
     if (!ok) {
         if (tid == 0) atomicExch(a.err, 7);

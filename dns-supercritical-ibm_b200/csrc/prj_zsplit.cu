@@ -63,10 +63,13 @@ __global__ void __launch_bounds__(256, PRJ_FFT_MINB) k_zfft(const ZfftArgs a) {
         }
     }
     __syncthreads();
-    if (DIR < 0) inplace_rows<-1, false, true>(zs, nr, a.nz, a.f, a.tw);
-    else inplace_rows<+1, true, true>(zs, nr, a.nz, a.f, a.tw);
     T* dst = static_cast<T*>(a.X) + row0 * a.nz;
-    for (int i = tid; i < tot; i += nthr) from_d2(dst[i], zs[sidx<true>(i)]);
+    if constexpr (DIR < 0) {
+        inplace_rows<-1, false, true>(zs, nr, a.nz, a.f, a.tw);
+        for (int i = tid; i < tot; i += nthr) from_d2(dst[i], zs[sidx<true>(i)]);
+    } else {
+        dit_rows_to<+1>(zs, nr, a.nz, a.f, a.tw, RowStore<T>{dst, (size_t)a.nz});
+    }
 }
 
 // the same by the out-of-place Stockham stages (any prime factor up to 64), natural order

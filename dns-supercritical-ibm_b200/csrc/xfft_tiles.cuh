@@ -302,10 +302,10 @@ __device__ __forceinline__ void fwd_xp_tile(const XArgs& a, unsigned char* sm, i
 // bwd_xp_tile: transposed load of X_k, X_{m-k} -> inverse split (scaled) into slot
 // order -> DIT passes -> P rows (x pairs as double2), optionally accumulated; the
 // tile's partial sum of P goes to psum[y][bx] (tiles_per_plane entries per plane).
-// EXTRAS = false: plain P = result (no accumulation, partial sums or norms), the form of
-// the persistent batch kernel.  STAGED: the spectrum comes from S (staged as above), and
+// EX = 0: plain P = result, the form of the FP64 solves; 1: also the partial sums; 2: P += result,
+// with the partial sums and the norms that are asked for.  STAGED: the spectrum comes from S (staged as above), and
 // after_split() is called once S is no longer read.
-template <class PL, bool EXTRAS = true, bool STAGED = false, class Hook = NoHook>
+template <class PL, int EX, bool STAGED = false, class Hook = NoHook>
 __device__ __forceinline__ void bwd_xp_tile(const XArgs& a, unsigned char* sm, int bx, int by, int tiles_per_plane,
                                             const double2* S = nullptr, Hook after_split = Hook{}) {
     double2* A = reinterpret_cast<double2*>(sm);
@@ -372,24 +372,25 @@ __device__ __forceinline__ void bwd_xp_tile(const XArgs& a, unsigned char* sm, i
     };
     double2* out = reinterpret_cast<double2*>(a.Pout) + ((size_t)y * a.nz + z0) * m;
     double sq0 = 0.0, sq1 = 0.0, ps = 0.0;
-    if constexpr (!EXTRAS) {
-        inverse([&](int r, int e, double2 v) { out[(size_t)r * m + e] = v; });
+    if constexpr (EX == 0) {
+        if constexpr (PL::n > 0) inverse([&](int r, int e, double2 v) { out[(size_t)r * m + e] = v; });
+        else dit_rows_to<+1>(A, nr, rs, a.f, a.tw, RowStore<double2>{out, (size_t)m});
         return;
-    }
-    inverse([&](int r, int e, double2 v) {
-        double2* o = out + (size_t)r * m + e;
-        if (a.accum) {
-            const double2 old = *o;
-            const double2 nv = make_double2(old.x + v.x, old.y + v.y);
+    } else if constexpr (EX == 1) {
+        inverse([&](int r, int e, double2 v) {
+            ps += v.x + v.y;
+            out[(size_t)r * m + e] = v;
+        });
+    } else {
+        inverse([&](int r, int e, double2 v) {
+            double2* o = out + (size_t)r * m + e;
+            const double2 old = *o, nv = make_double2(old.x + v.x, old.y + v.y);
             sq0 += v.x * v.x + v.y * v.y;
             sq1 += nv.x * nv.x + nv.y * nv.y;
             ps += nv.x + nv.y;
             *o = nv;
-        } else {
-            ps += v.x + v.y;
-            *o = v;
-        }
-    });
+        });
+    }
     if (a.psum) {
         // the tile's sum in a fixed order (per thread, then warp butterfly, then warps in order)
         __shared__ double wsum[8];  // warps of at most 256 threads
@@ -402,7 +403,7 @@ __device__ __forceinline__ void bwd_xp_tile(const XArgs& a, unsigned char* sm, i
             a.psum[(size_t)y * tiles_per_plane + bx] = t;
         }
     }
-    if (a.sq) {
+    if (EX == 2 && a.sq) {
         for (int o = 16; o > 0; o >>= 1) {
             sq0 += __shfl_xor_sync(0xffffffffu, sq0, o);
             sq1 += __shfl_xor_sync(0xffffffffu, sq1, o);
@@ -431,7 +432,7 @@ inline int x_box_k(int m) {
 // {2 tz, box_k, 1}; FP64 rows only) -- while the current tile runs its FFT passes and stores.
 // The tiles compute as fwd_xp_tile<2> / bwd_xp_tile<STAGED>, so the results are those of the
 // one-tile kernels.  A wait that runs out raises *err (6) and ends the run.
-template <class PL, bool FWD, bool EXTRAS>
+template <class PL, bool FWD>
 __device__ __forceinline__ void x_tiles_tma(const XArgs& a, const void* xmap, int tpp, int boxes, int box_k,
                                             unsigned char* sm, int soff, int sbytes, int first, int stride, int end,
                                             int* err) {
@@ -478,7 +479,7 @@ __device__ __forceinline__ void x_tiles_tma(const XArgs& a, const void* xmap, in
         // (the next iteration's barrier orders this tile's reads of its area before the next
         // tile's writes)
         if constexpr (FWD) fwd_xp_tile<2, PL>(a, sm, t % tpp, t / tpp, S, next);
-        else bwd_xp_tile<PL, EXTRAS, true>(a, sm, t % tpp, t / tpp, tpp, S, next);
+        else bwd_xp_tile<PL, 0, true>(a, sm, t % tpp, t / tpp, tpp, S, next);
     }
     __syncthreads();
     if (tid == 0) mbar_inval(bar);
