@@ -262,7 +262,7 @@ cudaError_t batchk_build(prj_plan* const* plans, double* const* d_P, int ncases,
         // their staged input, within kStagedBytes, so six CTAs fit per SM whatever the
         // plans' own tuning; a tile's shape does not change its results
         const int m = pl->fx64.m;
-        c.x.tz = std::min(c.x.tz, choose_tz_xp(m));
+        c.x.tz = c.x.tz == choose_tz_xp(m) ? fit_tz_xp(m) : std::min(c.x.tz, fit_tz_xp(m));
         while (c.x.tz > 1 && pass_x_smem(m, c.x.tz) + x_stage_bytes(m, c.x.tz) > kStagedBytes) c.x.tz /= 2;
         c.soff = (int)pass_x_smem(m, c.x.tz);
         c.xboxes = x_boxes(m);

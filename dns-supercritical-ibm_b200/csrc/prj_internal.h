@@ -205,6 +205,7 @@ inline cudaError_t launch_fwd_x_range(const prj_plan* pl, const double* Uh, cons
 }
 int choose_tz_xd(int m, bool even);
 int choose_tz_xp(int m);                 // rows per CTA of the pass-plan x kernels
+int fit_tz_xp(int m);                    // the most rows per CTA that fit
 size_t pass_x_smem(int m, int tz);       // their shared memory
 
 // z direction as separate kernels (prj_zsplit.cu)

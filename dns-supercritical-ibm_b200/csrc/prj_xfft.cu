@@ -293,12 +293,25 @@ cudaError_t allow_smem(K kernel, size_t bytes) {
 // CTAs per y plane of the pass-plan inverse x kernel (the width of its partial sums)
 int bwd_tiles_per_plane(const prj_plan* pl) { return (pl->g.nz + pl->tz_xp - 1) / pl->tz_xp; }
 
-// rows per CTA of the pass-plan x kernels: a power of two up to 16 whose padded rows
-// (stride pass_row_stride(m)) fit 32 KB, so that 6 CTAs share an SM; for the plans from m = 768,
-// where that is two rows, 64 KB and 256 threads
+// rows per CTA of the tiled x kernels: a power of two whose padded rows (stride
+// pass_row_stride(m)) fit 32 KB, so that 6 CTAs share an SM; for the plans from m = 768, where
+// that is two rows, 64 KB and 256 threads.  Up to 16 rows for lengths without a plan and
+// m <= 32, 8 for m <= 96 and 4 above: registers hold an SM to six CTAs whatever their size, so
+// smaller tiles spread a small grid over more SMs and shorten the last wave, down to 4 rows,
+// whose 64-byte runs of the transposed spectrum still make whole DRAM accesses.  Measured
+// (us per call, 16 / 8 / 4 / 2 rows): Poisson 128x96x64 41.1 / 37.1 / 39.8 / 45.2; step
+// 96x32x256 46.9 / 45.0 / 47.1 / 53.8, 256x128x128 190 / 162.3 / 160.6 / 169, 384x192x192
+// 567 / 473 / 459 / 494, 512x256x256 1323 / 1119 / 1058 / 1050; lengths without a plan 86.3 / 90.1 /
+// 92.4 / 99.8 at 160x80x100.
 int choose_tz_xp(int m) {
+    return std::min(fit_tz_xp(m), pass_orders(m) == 0 || m <= 32 ? 16 : m <= 96 ? 8 : 4);
+}
+
+// the most rows that fit (the persistent batch kernel's tiles, whose CTAs take many in a row)
+int fit_tz_xp(int m) {
+    const bool plan = pass_orders(m) > 0;
     int tz = 16;
-    const size_t most = (size_t)(pass_orders(m) > 0 ? x_threads(m) / kPassThreads : 1) * 32 * 1024;
+    const size_t most = (size_t)(plan ? x_threads(m) / kPassThreads : 1) * 32 * 1024;
     while (tz > 1 && (size_t)padded_len(tz * pass_row_stride(m), true) * sizeof(double2) > most) tz /= 2;
     return tz;
 }
