@@ -390,7 +390,7 @@ int run_mixed_core(prj_plan* pl, const double* Uh, const double* Vh, const doubl
         }
         {
             // the residual formed inside the forward x transform (no round trip of r through
-            // HBM), or as its own kernel where the x length has no pass plan
+            // HBM), or as its own kernel where nx is odd
             StageTimer tm(pl, prj::kStFwdX, st);
             const cudaError_t e = prj::launch_fwd_residual(pl, b, P, pl->pbar, st);
             if (e == cudaErrorNotSupported) {
@@ -1172,7 +1172,7 @@ int prj_plan_schedule(const prj_plan* plan, int mode, int* launches) {
     } else {
         // forward x, z transforms of the FP64 and FP32 rows, one Thomas launch, inverse z of both,
         // inverse x; per refinement pass also the plane means and a norm reset, and the
-        // residual where the forward x transform does not form it (no pass plan for nx/2);
+        // residual where the forward x transform does not form it (odd nx);
         // then the correction
         const int solve = 1 + 2 + 1 + 2 + 1;
         *launches = solve + plan->mixed_iters * (solve + (x_pass_active(plan) ? 2 : 3)) + 1;

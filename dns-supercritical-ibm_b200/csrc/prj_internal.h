@@ -194,7 +194,7 @@ bool zline_supported(const prj_plan* pl);  // launch_zline would run (not fall b
 cudaError_t launch_fwd_xd(const prj_plan* pl, FwdSource src, const double* P, const double* Uh, const double* Vh,
                           const double* Wh, const StepScalars* sc, cudaStream_t st, double* bout = nullptr,
                           YRange yr = YRange{});
-// psum: per-CTA sums of the written P, [y][tile] (pass-plan kernel only; otherwise
+// psum: per-CTA sums of the written P, [y][tile] (tiled kernel only; otherwise
 // cudaErrorNotSupported and nothing launched)
 cudaError_t launch_bwd_xd(const prj_plan* pl, double* P, cudaStream_t st, int accum = 0, double* sq = nullptr,
                           YRange yr = YRange{}, double* psum = nullptr);
@@ -221,8 +221,8 @@ cudaError_t launch_plane_mean(const prj_plan* pl, const double* P, double* pbar,
 // plane means from the inverse x kernel's partial sums ([ny][tiles])
 cudaError_t launch_plane_mean_partials(const prj_plan* pl, const double* psum, int tiles, double* pbar,
                                        cudaStream_t st);
-// forward x transform of the residual B - A P formed on the fly (the pass-plan kernel);
-// cudaErrorNotSupported when the x length has no pass plan or an array is not 16-byte
+// forward x transform of the residual B - A P formed on the fly (the tiled kernel);
+// cudaErrorNotSupported when nx is odd or an array is not 16-byte
 // aligned (the caller then runs launch_residual and the forward x of its result)
 cudaError_t launch_fwd_residual(const prj_plan* pl, const double* B, const double* P, const double* pbar,
                                 cudaStream_t st);

@@ -439,7 +439,7 @@ cudaError_t launch_bwd_xd(const prj_plan* pl, double* P, cudaStream_t st, int ac
         const cudaError_t e2 = launch_xpass(pl, false, FwdSource::Pressure, a, yr.y1 - yr.y0, st);
         if (e2 != cudaErrorNotSupported) return e2;
     }
-    if (psum) return cudaErrorNotSupported;  // partial sums come from the pass-plan kernel only
+    if (psum) return cudaErrorNotSupported;  // partial sums come from the tiled kernel only
     const size_t smem = smem_bytes(a);
     cudaError_t e = allow_smem(k_bwd_xd, smem);
     if (e != cudaSuccess) return e;
