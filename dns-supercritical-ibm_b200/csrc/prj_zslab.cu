@@ -165,7 +165,9 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_zslab(const __grid_constant__ 
             }
         }
     }
-    // this thread's lines
+    // this thread's lines.  A slot past n holds none: its values are zeros that no shared-memory
+    // read supplies (the cells of the lines change under their own threads' sweeps, between
+    // barriers), and a thread without a line takes no part in the sweeps.
     int at[LPT], piv[LPT], slot[LPT];
 #pragma unroll
     for (int q = 0; q < LPT; q++) {
@@ -218,8 +220,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_zslab(const __grid_constant__ 
     if (ok) {
         const uint32_t up = c < C - 1 ? cluster_map(carry, (uint32_t)(c + 1)) : 0u;
         const uint32_t upbar = c < C - 1 ? cluster_map(&bars[1], (uint32_t)(c + 1)) : 0u;
-        // lines past n run along on line 0's values and store nothing; the loads of a block
-        // are issued a block ahead
+        // the loads of a block are issued a block ahead
         constexpr int B = slab_up(LPT);
         double2 below[LPT];
 #pragma unroll
@@ -237,7 +238,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_zslab(const __grid_constant__ 
 #pragma unroll
                 for (int u = 0; u < B; u++) {
                     const int r = min(r0 + u, nr - 1);
-                    k.v[q][u] = buf[at[q] + r * rp];
+                    k.v[q][u] = slot[q] < n ? buf[at[q] + r * rp] : make_double2(0.0, 0.0);
                     k.a[q][u] = abuf[(kx == 0 && piv[q] == 0 ? H : 0) + r];
                 }
             }
@@ -251,13 +252,15 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_zslab(const __grid_constant__ 
                 for (int u = 0; u < B; u++)
                     if (u < nb && slot[q] < n) buf[at[q] + (r0 + u) * rp] = k.v[q][u];
         };
-        load(even, 0);
-        for (int r0 = 0; r0 < nr; r0 += 2 * B) {
-            load(odd, min(r0 + B, nr - 1) / B * B);
-            sweep(even, r0);
-            if (r0 + B >= nr) break;
-            load(even, min(r0 + 2 * B, nr - 1) / B * B);
-            sweep(odd, r0 + B);
+        if (slot[0] < n) {
+            load(even, 0);
+            for (int r0 = 0; r0 < nr; r0 += 2 * B) {
+                load(odd, min(r0 + B, nr - 1) / B * B);
+                sweep(even, r0);
+                if (r0 + B >= nr) break;
+                load(even, min(r0 + 2 * B, nr - 1) / B * B);
+                sweep(odd, r0 + B);
+            }
         }
         // a quotient that may differ: the rows again from memory, which still holds them, and
         // the sweep by plain division
@@ -269,11 +272,12 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_zslab(const __grid_constant__ 
             FFT::forward(buf, nr, rs, a);
 #pragma unroll
             for (int q = 0; q < LPT; q++) {
+                if (slot[q] >= n) continue;
                 prev[q] = below[q];
                 for (int r = 0; r < nr; r++) {
                     prev[q] = step_up_safe(buf[at[q] + r * rp], dbuf[piv[q] + r],
                                            abuf[(kx == 0 && piv[q] == 0 ? H : 0) + r], prev[q]);
-                    if (slot[q] < n) buf[at[q] + r * rp] = prev[q];
+                    buf[at[q] + r * rp] = prev[q];
                 }
             }
         }
@@ -325,7 +329,8 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_zslab(const __grid_constant__ 
             for (int q = 0; q < LPT; q++) {
                 slab_planes_of<B>(k.f[q], dbuf + piv[q] + r0);
 #pragma unroll
-                for (int u = 0; u < B; u++) k.v[q][u] = buf[at[q] + min(r0 + u, nr - 1) * rp];
+                for (int u = 0; u < B; u++)
+                    k.v[q][u] = slot[q] < n ? buf[at[q] + min(r0 + u, nr - 1) * rp] : make_double2(0.0, 0.0);
             }
         };
         auto sweep = [&](Block& k, int r0) {
@@ -337,7 +342,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_zslab(const __grid_constant__ 
                 for (int u = 0; u < B; u++)
                     if (u < nb && slot[q] < n) buf[at[q] + (r0 + u) * rp] = k.v[q][u];
         };
-        if (top >= 0) {
+        if (top >= 0 && slot[0] < n) {
             int r0 = top / B * B;
             load(even, r0);
             for (; r0 >= 0; r0 -= 2 * B) {

@@ -197,7 +197,8 @@ __device__ __forceinline__ void zline_tile(const ZLineArgs& a, const void* tmap,
         cphase[d] ^= 1u;
         if (__syncthreads_or(!ok)) return false;
 #pragma unroll
-        for (int q = 0; q < LPT; q++) prev[q] = carry[d * n + at[q]];
+        for (int q = 0; q < LPT; q++)
+            if (slot[q] < n) prev[q] = carry[d * n + slot[q]];
         left[d]--;
         if (tid == 0 && left[d] > 0) mbar_arrive_expect_tx(&bars[NS + d], carry_bytes);
         return true;
@@ -252,9 +253,9 @@ __device__ __forceinline__ void zline_tile(const ZLineArgs& a, const void* tmap,
                 return;
             }
         }
-        // plane by plane (lines past n run along on line 0's values and store nothing); a
-        // quotient that may differ is noticed at the end of the chunk, whose inputs the stage
-        // still holds
+        // plane by plane (lines past n run along on line 0's values, which no thread changes in
+        // this phase, and store nothing); a quotient that may differ is noticed at the end of the
+        // chunk, whose inputs the stage still holds
         double2 below[LPT];
 #pragma unroll
         for (int q = 0; q < LPT; q++) below[q] = prev[q];
