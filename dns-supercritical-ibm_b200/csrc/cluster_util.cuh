@@ -48,4 +48,15 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t phase,
     }
 }
 
+// The way out of a CTA that gave up a wait (every thread calls it): its own copy on `copy_bar`
+// (phase 0; null: none was issued) must not land after it has left, so thread 0 waits for that
+// within the limit first; then the cluster barrier, so that no CTA leaves while a neighbour can
+// still write to it.
+__device__ __forceinline__ void cluster_leave(uint64_t* copy_bar) {
+    if (copy_bar && threadIdx.x == 0) mbar_wait_bounded(copy_bar, 0);
+    __syncthreads();
+    cluster_arrive();
+    cluster_wait();
+}
+
 }  // namespace prj

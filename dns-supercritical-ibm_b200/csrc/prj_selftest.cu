@@ -4,9 +4,12 @@
 // a limit: after a clock budget a wait gives up, the kernel raises an error word
 // and returns, and the host reports PRJ_ERR_TIMEOUT with the context intact.
 // prj_selftest_wait_timeout exercises that path on purpose without any fault: one
-// thread waits, with a short budget, on an mbarrier that nothing arrives on.
+// thread waits, with a short budget, on an mbarrier that nothing arrives on; and the two
+// CTAs of a cluster, as those of the z kernels, wait for a carry that no neighbour sends
+// while a copy of their own is under way, and leave together.
 #include "../../include/projection.h"
 #include "prj_internal.h"
+#include "cluster_util.cuh"
 #include "div_rn.cuh"
 #include "tma_util.cuh"
 
@@ -22,6 +25,36 @@ __global__ void k_wait_selftest(long long budget, int* err) {
     __syncthreads();
     const bool ok = mbar_wait_bounded(&bar, 0, budget);
     if (__syncthreads_or(!ok) && threadIdx.x == 0) atomicExch(err, 3);
+}
+
+// src: kClusterCopy bytes; err[rank]: 3 when the wait gave up and the copy had landed by the
+// time the CTA could leave
+constexpr int kClusterCopy = 4096;
+__global__ void __launch_bounds__(64) __cluster_dims__(2, 1, 1)
+    k_cluster_wait_selftest(long long budget, const unsigned* src, int* err) {
+    __shared__ uint64_t bars[2];  // [0] the copy, [1] the carry
+    __shared__ __align__(128) unsigned rows[kClusterCopy / sizeof(unsigned)];
+    const int rank = (int)cluster_rank();
+    if (threadIdx.x == 0) {
+        mbar_init(&bars[0], 1);
+        mbar_init(&bars[1], 1);
+        mbar_fence_init();
+        mbar_arrive_expect_tx(&bars[1], 16);  // bytes that no neighbour sends
+    }
+    __syncthreads();
+    cluster_arrive();
+    if (threadIdx.x == 0) {
+        mbar_arrive_expect_tx(&bars[0], kClusterCopy);
+        bulk_g2s(rows, src, kClusterCopy, &bars[0]);
+    }
+    cluster_wait();
+    const bool ok = mbar_wait_cluster(&bars[1], 0, budget);
+    const bool gave_up = __syncthreads_or(!ok);
+    cluster_leave(&bars[0]);
+    bool landed = mbar_try_wait(&bars[0], 0);
+    for (int i = threadIdx.x; i < kClusterCopy / (int)sizeof(unsigned); i += blockDim.x)
+        landed = landed && rows[i] == 0xabababab;
+    if (!__syncthreads_or(!(gave_up && landed)) && threadIdx.x == 0) atomicExch(err + rank, 3);
 }
 
 // splitmix64: a reproducible stream of 64-bit words per index
@@ -148,18 +181,22 @@ extern "C" int prj_selftest_wait_timeout(int device, long long budget_cycles) {
     int prev = 0;
     cudaGetDevice(&prev);
     cudaError_t e = cudaSetDevice(device);
-    int* d_err = nullptr;
-    int h_err = 0;
-    if (e == cudaSuccess) e = cudaMalloc((void**)&d_err, sizeof(int));
-    if (e == cudaSuccess) e = cudaMemset(d_err, 0, sizeof(int));
+    // the three error words, then (128 bytes on) the source of the copies
+    unsigned char* d_buf = nullptr;
+    int h_err[3] = {0, 0, 0};
+    if (e == cudaSuccess) e = cudaMalloc((void**)&d_buf, 128 + prj::kClusterCopy);
+    if (e == cudaSuccess) e = cudaMemset(d_buf, 0, 128);
+    if (e == cudaSuccess) e = cudaMemset(d_buf + 128, 0xab, prj::kClusterCopy);
     if (e == cudaSuccess) {
+        int* d_err = reinterpret_cast<int*>(d_buf);
         prj::k_wait_selftest<<<1, 32>>>(budget_cycles, d_err);
+        prj::k_cluster_wait_selftest<<<2, 64>>>(budget_cycles, reinterpret_cast<const unsigned*>(d_buf + 128), d_err + 1);
         e = cudaGetLastError();
     }
-    if (e == cudaSuccess) e = cudaMemcpy(&h_err, d_err, sizeof(int), cudaMemcpyDeviceToHost);
-    if (d_err) cudaFree(d_err);
+    if (e == cudaSuccess) e = cudaMemcpy(h_err, d_buf, sizeof(h_err), cudaMemcpyDeviceToHost);
+    if (d_buf) cudaFree(d_buf);
     cudaSetDevice(prev);
     if (e != cudaSuccess) return prj::record_error(PRJ_ERR_CUDA, cudaGetErrorString(e));
-    if (h_err) return prj::record_error(PRJ_ERR_TIMEOUT, "bounded device wait gave up (as intended by the self-test)");
+    if (h_err[0] && h_err[1] && h_err[2]) return prj::record_error(PRJ_ERR_TIMEOUT, "bounded device wait gave up (as intended by the self-test)");
     return PRJ_OK;
 }

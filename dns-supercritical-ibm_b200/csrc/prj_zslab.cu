@@ -21,8 +21,8 @@
 // c_y / D_y correctly rounded as tabulated there), so the results are the same bits.
 //
 // Every wait on an mbarrier is bounded (a clock budget); a CTA whose wait runs out raises
-// the plan's error word and leaves through the cluster barrier, so that no CTA exits while
-// a neighbour can still write to its shared memory.  In the ordinary path a CTA's last
+// the plan's error word, waits (bounded) for its own row copy and leaves through the cluster
+// barrier, so that no CTA exits while a neighbour can still write to its shared memory.  In the ordinary path a CTA's last
 // incoming stores are the ones it has waited for.
 #include <cuda.h>
 
@@ -363,8 +363,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_zslab(const __grid_constant__ 
     }
     if (!ok) {
         if (tid == 0) atomicExch(a.err, 7);
-        cluster_arrive();
-        cluster_wait();
+        cluster_leave(a.tma ? &bars[0] : nullptr);
     }
 }
 

@@ -221,10 +221,7 @@ __device__ __forceinline__ void zline_tile(const ZLineArgs& a, const void* tmap,
         if (tid == 0)
 #pragma unroll
             for (int s = 0; s < NS; s++) mbar_inval(&bars[s]);
-        if constexpr (CL) {  // no CTA leaves while a neighbour can still write to it
-            cluster_arrive();
-            cluster_wait();
-        }
+        if constexpr (CL) cluster_leave(nullptr);
     };
 
 #pragma unroll

@@ -353,9 +353,10 @@ int prj_plan_set_tuning(prj_plan* plan, const prj_tuning* tuning);
 
 /* Diagnostic of the bounded device-side waits of the pipelined kernels: one
  * kernel waits, for at most budget_cycles SM clock cycles, on an mbarrier that
- * nothing arrives on, gives up, and reports it.  Returns PRJ_ERR_TIMEOUT when the
- * wait gave up as designed (the context stays usable), PRJ_OK if it unexpectedly
- * completed.  No fault, trap or unbounded wait is involved. */
+ * nothing arrives on, gives up, and reports it; the two CTAs of a cluster do the
+ * same with a copy of their own under way, wait for that copy and leave together.
+ * Returns PRJ_ERR_TIMEOUT when every wait gave up as designed (the context stays
+ * usable), PRJ_OK if one did not.  No fault, trap or unbounded wait is involved. */
 int prj_selftest_wait_timeout(int device, long long budget_cycles);
 
 /* Diagnostic of the division the Thomas forward sweeps use: n pseudo-random pairs

@@ -1,6 +1,7 @@
 """The bounded device waits give up and report instead of hanging: a wait on an mbarrier that
-nothing arrives on (budget ~1 ms of SM clock) must come back as PRJ_ERR_TIMEOUT, and the context
-must stay usable for the next solve."""
+nothing arrives on (budget ~1 ms of SM clock), and the wait of each CTA of a cluster for a carry
+that its neighbour never sends, with a copy of its own in flight that has to land before the CTA
+leaves, must come back as PRJ_ERR_TIMEOUT, and the context must stay usable for the next solve."""
 import numpy as np
 import pytest
 

@@ -57,6 +57,18 @@ def test_slab_equals_split(cuda_device, shape, planes):
     np.testing.assert_array_equal(got, want)
 
 
+# threads without a line, and (270, 288) threads with a second line and without; half of the planes
+# far below the division's window
+@pytest.mark.parametrize("nz", [2, 9, 32, 96, 225, 250, 270, 288])
+def test_slots_without_a_line(cuda_device, nz):
+    nx, ny = 16, 24
+    rhs = _rhs(nx, ny, nz, 4)
+    rhs[:, :, : ny // 2] *= 2.0 ** -1000
+    got, want, launches = _both(nx, ny, nz, rhs)
+    assert launches == 4
+    np.testing.assert_array_equal(got, want)
+
+
 # clusters of two to eight CTAs, chunks cut short at the top, more wavenumbers than SMs
 @pytest.mark.parametrize("shape", [(256, 128, 128), (256, 67, 128), (300, 130, 192), (200, 150, 256), (128, 97, 384),
                                    (330, 200, 64), (64, 130, 256), (150, 60, 96)])
