@@ -121,7 +121,7 @@ constexpr int kZlStages = 2;
 __host__ __device__ constexpr int batch_lpt(int n) { return (n + kBatchThreads - 1) / kBatchThreads; }
 template <class PL>
 __device__ __noinline__ void tile_zline(const BatchCaseDev& c, const CUtensorMap* tmap, int kx, unsigned char* sm) {
-    zline_tile<PL, kZlStages, batch_lpt(PL::n), kBatchThreads, 1>(c.zl, tmap, kx, sm);
+    zline_tile<PL, kZlStages, batch_lpt(PL::n), kBatchThreads, 1, false, true>(c.zl, tmap, kx, sm);
 }
 
 __device__ __forceinline__ void run_x_fwd(const BatchCaseDev& c, const CUtensorMap* xmap, int t0, int count,

@@ -92,12 +92,29 @@ PRJ_PASS_PLANS(PRJ_ZL_LAYOUT_CHECK)
 // (the 9th out of bounds, zero-filled) writes.
 __host__ __device__ inline size_t zl_slot_bytes(int n, int yb) { return ((size_t)yb * n * 18 + 127) / 128 * 128; }
 
+// the forward sweep of one line's nr planes of a chunk again, by plain division: d_y in the
+// stage's rows, d' to x (plane stride xs) and returned
+template <int n>
+__device__ __forceinline__ double2 zline_redo(double2* x, size_t xs, const double2* buf, int slot, const double* D, int mzs,
+                                              const double* av, bool first, int nr, double2 prev) {
+    for (int r = 0; r < nr; r++) {
+        prev = step_up_safe(buf[sidx<true>(r * n + slot)], D[(size_t)r * mzs], first && r == 0 ? 0.0 : av[r], prev);
+        x[r * xs] = prev;
+    }
+    return prev;
+}
+template <int n>
+__device__ __noinline__ double2 zline_redo_call(double2* x, size_t xs, const double2* buf, int slot, const double* D, int mzs,
+                                                const double* av, bool first, int nr, double2 prev) {
+    return zline_redo<n>(x, xs, buf, slot, D, mzs, av, first, nr, prev);
+}
+
 // The z solve of x wavenumber kx: NT threads (the CTA), LPT lines per thread (NT LPT >=
 // n; slots past n idle in the Thomas phase), NS stages of a.yb planes in `zsm`
 // (zline_smem bytes).  Each stage's rows arrive by one tensor-map copy (`tmap`:
 // zline_tmap's 4-D view of the spectrum) issued by thread 0 and completed on an mbarrier;
 // the pivot rows are cp.async copies (their pieces are permuted).  UP planes of the forward
-// sweep are unrolled.  Every mbarrier wait is bounded: on a timeout the tile raises *a.err,
+// sweep are unrolled; CALL: the redo of a line is a call.  Every mbarrier wait is bounded: on a timeout the tile raises *a.err,
 // waits (bounded) for its copies in flight and returns.
 //
 // CL: the CTAs of a cluster of a.C share the wavenumber, CTA c taking the chunks c, c + C, ...
@@ -105,7 +122,7 @@ __host__ __device__ inline size_t zl_slot_bytes(int n, int yb) { return ((size_t
 // way down) goes to the next chunk's CTA by st.async into its carry row, completed on its
 // mbarrier; copies, transforms and the pivots' reciprocals (rbuf) of C chunks run meanwhile.
 // One carry row per direction is enough: the next carry depends on this CTA's own.
-template <class PL, int NS, int LPT, int NT, int UP = 2, bool CL = false>
+template <class PL, int NS, int LPT, int NT, int UP = (LPT > 1 ? 1 : 2), bool CL = false, bool CALL = false>
 __device__ __forceinline__ void zline_tile(const ZLineArgs& a, const void* tmap, int kx, unsigned char* zsm) {
     constexpr int n = PL::n;
     static_assert(NT * LPT >= n, "every line has a thread");
@@ -141,14 +158,16 @@ __device__ __forceinline__ void zline_tile(const ZLineArgs& a, const void* tmap,
     uint32_t phase = 0;    // bit s: parity of stage s's next completion
     uint32_t pending = 0;  // bit s: stage s has a copy in flight (the same in every thread)
 
-    // this thread's lines
-    int slot[LPT], at[LPT], kzs[LPT];
+    // this thread's lines; a slot past n (none where the threads' slots are the lines exactly)
+    // holds no line
+    constexpr bool kExact = NT * LPT == n;
+    auto line = [&](int q) { return kExact || tid + q * NT < n; };
+    int slot[LPT], kzs[LPT];
     bool is00[LPT];
 #pragma unroll
     for (int q = 0; q < LPT; q++) {
         slot[q] = tid + q * NT;
-        at[q] = slot[q] < n ? slot[q] : 0;
-        const int kz = a.kz_of_slot[at[q]];
+        const int kz = a.kz_of_slot[line(q) ? slot[q] : 0];
         const int kf = kz <= n - kz ? kz : n - kz;
         kzs[q] = 2 * zl_piece(kf >> 1) + (kf & 1);  // position in a shared pivot row
         is00[q] = (kx == 0 && kz == 0);
@@ -198,7 +217,7 @@ __device__ __forceinline__ void zline_tile(const ZLineArgs& a, const void* tmap,
         if (__syncthreads_or(!ok)) return false;
 #pragma unroll
         for (int q = 0; q < LPT; q++)
-            if (slot[q] < n) prev[q] = carry[d * n + slot[q]];
+            if (line(q)) prev[q] = carry[d * n + slot[q]];
         left[d]--;
         if (tid == 0 && left[d] > 0) mbar_arrive_expect_tx(&bars[NS + d], carry_bytes);
         return true;
@@ -207,7 +226,7 @@ __device__ __forceinline__ void zline_tile(const ZLineArgs& a, const void* tmap,
         const uint32_t row = cluster_map(carry + d * n, (uint32_t)to), bar = cluster_map(&bars[NS + d], (uint32_t)to);
 #pragma unroll
         for (int q = 0; q < LPT; q++)
-            if (slot[q] < n) st_async(row + (uint32_t)slot[q] * 16u, prev[q], bar);
+            if (line(q)) st_async(row + (uint32_t)slot[q] * 16u, prev[q], bar);
     };
     auto bail = [&]() {
         if (tid == 0) {
@@ -250,42 +269,53 @@ __device__ __forceinline__ void zline_tile(const ZLineArgs& a, const void* tmap,
                 return;
             }
         }
-        // plane by plane (lines past n run along on line 0's values, which no thread changes in
-        // this phase, and store nothing); a quotient that may differ is noticed at the end of the
-        // chunk, whose inputs the stage still holds
-        double2 below[LPT];
-#pragma unroll
-        for (int q = 0; q < LPT; q++) below[q] = prev[q];
+        // plane by plane; a quotient that may differ is noticed at the end of the chunk, whose
+        // inputs the stage still holds.  A slot without a line carries zeros.
         unsigned outside = 0;
 #pragma unroll UP
         for (int r = 0; r < nr; r++) {
-            double2 v[LPT][1];
-            double D[LPT][1], rD[LPT][1], av[LPT][1];
-#pragma unroll
-            for (int q = 0; q < LPT; q++) {
-                v[q][0] = buf[sidx<true>(r * n + at[q])];
-                D[q][0] = dbuf[(size_t)r * mzs + kzs[q]];
-                rD[q][0] = CL ? rbuf[(size_t)r * mzs + kzs[q]] : __drcp_rn(D[q][0]);  // off the chain
-                av[q][0] = y0 + r > 0 ? abuf[(is00[q] ? yb : 0) + r] : 0.0;
-            }
-            sweep_up<1, LPT>(v, D, rD, av, 1, prev, outside);
             double2* grow = a.X + ((size_t)(y0 + r) * nh + kx) * n;
+            // G lines at a time, more in flight spill.  Measured with the redo in the loop below
+            // and each line's d' carried to it (all lines at once, 1268 bytes of spills at
+            // n = 1536) and now: 406 -> 337 us at 592 x 24 x 1536, 380 -> 366 us at 592 x 64 x 768,
+            // 238 -> 219 us at 592 x 64 x 512, 938 -> 925 us at 768 x 384 x 384.  In the batch
+            // kernel, at 80 registers, the redo as a call: 2583 -> 2565 us for 64 cases; the other
+            // way round (an inlined redo there, a call here) 2595 and 953 us.
+            constexpr int G = LPT > 1 ? 2 : 1;
+            static_assert(LPT % G == 0, "whole groups of lines");
 #pragma unroll
-            for (int q = 0; q < LPT; q++)
-                if (slot[q] < n) grow[slot[q]] = v[q][0];
-        }
-        if (outside) {
+            for (int q0 = 0; q0 < LPT; q0 += G) {
+                double2 v[G][1], p[G];
+                double D[G][1], rD[G][1], av[G][1];
 #pragma unroll
-            for (int q = 0; q < LPT; q++) prev[q] = below[q];
-            for (int r = 0; r < nr; r++) {
-                double2* grow = a.X + ((size_t)(y0 + r) * nh + kx) * n;
+                for (int g = 0; g < G; g++) {
+                    const int q = q0 + g;
+                    p[g] = prev[q];
+                    v[g][0] = line(q) ? buf[sidx<true>(r * n + slot[q])] : make_double2(0.0, 0.0);
+                    D[g][0] = dbuf[(size_t)r * mzs + kzs[q]];
+                    rD[g][0] = CL ? rbuf[(size_t)r * mzs + kzs[q]] : __drcp_rn(D[g][0]);  // off the chain
+                    av[g][0] = y0 + r > 0 ? abuf[(is00[q] ? yb : 0) + r] : 0.0;
+                }
+                sweep_up<1, G>(v, D, rD, av, 1, p, outside);
 #pragma unroll
-                for (int q = 0; q < LPT; q++) {
-                    prev[q] = step_up_safe(buf[sidx<true>(r * n + at[q])], dbuf[(size_t)r * mzs + kzs[q]],
-                                           y0 + r > 0 ? abuf[(is00[q] ? yb : 0) + r] : 0.0, prev[q]);
-                    if (slot[q] < n) grow[slot[q]] = prev[q];
+                for (int g = 0; g < G; g++) {
+                    prev[q0 + g] = p[g];
+                    if (line(q0 + g)) grow[slot[q0 + g]] = v[g][0];
                 }
             }
+        }
+        if (outside) {
+            // from d' of the plane below: the carry row, which the next carry has not reached
+            // (hand_on follows), or the row that this thread stored
+            for (int q = 0; q < LPT; q++)
+                if (line(q)) {
+                    double2* x = a.X + ((size_t)y0 * nh + kx) * n + slot[q];
+                    double2 p = make_double2(0.0, 0.0);
+                    if (y0 > 0) p = CL ? carry[slot[q]] : *(x - (size_t)nh * n);
+                    const double *Dq = dbuf + kzs[q], *aq = abuf + (is00[q] ? yb : 0);
+                    if constexpr (CALL) prev[q] = zline_redo_call<n>(x, (size_t)nh * n, buf, slot[q], Dq, mzs, aq, y0 == 0, nr, p);
+                    else prev[q] = zline_redo<n>(x, (size_t)nh * n, buf, slot[q], Dq, mzs, aq, y0 == 0, nr, p);
+                }
         }
         if constexpr (CL)
             if (c + 1 < nch) hand_on(0, (rank + 1) % C);
@@ -321,7 +351,7 @@ __device__ __forceinline__ void zline_tile(const ZLineArgs& a, const void* tmap,
             const int y = y0 + r;
 #pragma unroll
             for (int q = 0; q < LPT; q++) {
-                if (slot[q] < n) {
+                if (line(q)) {
                     double2& cell = buf[sidx<true>(r * n + slot[q])];
                     const double2 d = cell;
                     if (y == ny - 1) {

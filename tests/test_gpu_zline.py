@@ -116,3 +116,35 @@ def test_line_kernel_outside_the_fast_division_window(cuda_device, monkeypatch, 
     if scale == 2.0 ** -960:  # normal inputs: the oracle's plain division agrees closely
         Po, _ = oracle.poisson(rhs, dx, dz, b6)
         assert np.linalg.norm(out["line"] - Po) <= 1e-12 * np.linalg.norm(Po)
+
+
+@pytest.mark.parametrize("nz", [48, 192, 256, 384, 512, 768, 1024, 1536])
+def test_line_kernel_redoes_some_chunks(cuda_device, nz):
+    """The lower half of the planes outside the division's window: those chunks are redone, each
+    from the plane below it, and the chunks above are not; every number of lines per thread, and
+    the batch kernel's tiles."""
+    import prj
+    import workloads
+    nx, ny = 32, 37
+    rhs, yu, dx, dz = workloads.poisson_rhs(nx, ny, nz, seed=24)
+    rhs[:, :, : ny // 2] *= 2.0 ** -1000
+    rhs = np.asfortranarray(rhs)
+    b6 = prj.bands(yu, "consistent")
+    out = {}
+    for mode, tuning in (("split", dict(z_mode=0, z_rows=4)), ("line", dict(z_mode=3, z_planes=4, z_stages=2))):
+        with prj.Plan(nx, nz, ny, dx, dz, b6) as plan:
+            plan.set_tuning(**tuning)
+            assert plan.launches_per_step() == {"split": 6, "line": 4}[mode]
+            t = to_dev(rhs)
+            plan.poisson_fp64(t)
+            plan.check_error()
+            out[mode] = from_dev(t)
+    np.testing.assert_array_equal(out["split"], out["line"])
+    with prj.Plan(nx, nz, ny, dx, dz, b6) as plan:
+        t = to_dev(rhs)
+        with prj.Batch([plan], [t]) as batch:
+            assert batch.info["persistent"] or nz > 256
+            t.copy_(to_dev(rhs))  # creating the graph form solves once
+            batch.launch()
+            batch.check_error()
+        np.testing.assert_array_equal(from_dev(t), out["split"])
