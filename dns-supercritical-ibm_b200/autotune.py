@@ -3,7 +3,7 @@
 For one grid size it times candidate tunings of a plan (prj_tuning,
 include/projection.h) on an in-place FP64 solve with CUDA events, in two phases:
 first the launch shapes -- x-rows per CTA of the x transforms, spectral rows per
-CTA of the z transforms, split versus fused z kernels -- in the default radix
+CTA of the z transforms, z kernels picked by size, split or fused -- in the default radix
 orders; then, with the best shapes, every compiled radix order of the x and z
 transform lengths (the pass plans of fft_pass.cuh, where the reference lets
 FFTW/cuFFT pick a factorisation at plan time, poisson_solver_multigpu.f90:77-129).
@@ -47,7 +47,8 @@ def key(plan) -> str:
 
 
 def candidates(plan):
-    out = []
+    default = plan.tuning["z_mode"]
+    out = [dict(x_rows=x_rows, z_rows=0, z_mode=default, z_auto=True) for x_rows in (2, 4, 8, 16)]
     for z_mode in (0, 1, 3):
         for x_rows in (2, 4, 8, 16):
             for z_rows in ((0, 4, 8, 16) if z_mode == 0 else (0,)):
@@ -83,7 +84,7 @@ def time_solve(plan, P, reps):
     return e0.elapsed_time(e1) / reps
 
 
-FIELDS = ("x_rows", "z_rows", "z_mode", "x_order", "z_order")
+FIELDS = ("x_rows", "z_rows", "z_mode", "x_order", "z_order", "z_auto")
 
 
 def _apply(plan, t):
@@ -106,7 +107,7 @@ def tune(plan, reps: int = 5, use_cache: bool = True) -> dict:
     for phase in (0, 1):
         cands = candidates(plan) if phase == 0 else order_candidates(plan, {f: best[f] for f in FIELDS})
         for c in cands:
-            c = dict({"x_order": 0, "z_order": 0}, **c)
+            c = dict({"x_order": 0, "z_order": 0, "z_auto": False}, **c)
             try:
                 _apply(plan, c)
             except prj.PrjError:

@@ -442,7 +442,7 @@ int run_mixed_poisson(prj_plan* pl, double* P, cudaStream_t st) {
 // runtime-radix kernel per wavenumber, k_zsolve_pipe, took 346 us for 68 wavenumbers of 60
 // planes at nz = 77, where the three take 40)
 bool split_z(const prj_plan* pl) {
-    return pl->zmode == 0 || pl->zmode == 3 || (pl->zmode == 1 && pl->zmode_default == 1 && pl->z_planes == 0 && pl->z_stages == 0);
+    return pl->zmode == 0 || pl->zmode == 3 || (pl->zmode == 1 && pl->z_auto && pl->z_planes == 0 && pl->z_stages == 0);
 }
 
 // z transforms + Thomas: three kernels (split) or one fused kernel
@@ -1180,6 +1180,20 @@ int prj_plan_schedule(const prj_plan* plan, int mode, int* launches) {
     return PRJ_OK;
 }
 
+int prj_plan_set_z_auto(prj_plan* plan, int on) {
+    const int rc = check_plan(plan);
+    if (rc) return rc;
+    plan->z_auto = on != 0;
+    if (on) plan->zmode = plan->zmode_default;
+    return PRJ_OK;
+}
+
+int prj_plan_get_z_auto(const prj_plan* plan, int* on) {
+    if (!plan || !on) return fail(PRJ_ERR_ARG, "NULL argument");
+    *on = plan->z_auto ? 1 : 0;
+    return PRJ_OK;
+}
+
 int prj_plan_get_tuning(const prj_plan* plan, prj_tuning* out) {
     if (!plan || !out) return fail(PRJ_ERR_ARG, "NULL argument");
     out->x_rows = x_pass_active(plan) ? plan->tz_xp : plan->tz_xd;
@@ -1271,6 +1285,7 @@ int prj_plan_set_tuning(prj_plan* plan, const prj_tuning* t) {
     plan->tz_xp = t->x_rows;
     plan->zfft_rows = t->z_rows;
     plan->zmode = t->z_mode;
+    plan->z_auto = false;  // the caller names the z kernels (prj_plan_set_z_auto takes that back)
     plan->z_planes = t->z_planes;
     plan->z_stages = t->z_stages;
     plan->thomas_async = t->thomas_ring;

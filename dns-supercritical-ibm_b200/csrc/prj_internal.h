@@ -124,6 +124,8 @@ struct prj_plan {
     int zmode = 0;                // z direction: 0 split kernels, 1 fused pipelined, 2 unpipelined,
                                   // 3 one pass-plan kernel per x wavenumber (split where no plan)
     int zmode_default = 0;        // zmode as the plan was created
+    bool z_auto = true;           // the z kernels are picked by size (zmode is zmode_default); false
+                                  // once a tuning names them
     int sms = 0;                  // SMs of the plan's device
     bool use_pass = true;         // compile-time pass-plan FFT kernels where the length has one
     int thomas_async = -1;        // Thomas lines streamed through a cp.async shared-memory ring:

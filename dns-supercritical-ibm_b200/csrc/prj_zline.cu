@@ -137,7 +137,7 @@ static void zline_cluster_shape(const prj_plan* pl, int* C_out, int* yb_out) {
     *C_out = *yb_out = 0;
     const Geometry& g = pl->g;
     // a z kernel, row count, ring, chunk or stage count chosen by the plan's tuning stands
-    if (pl->zmode != pl->zmode_default || (pl->zmode != 0 && pl->zmode != 3) || pl->zfft_rows != 0 ||
+    if (!pl->z_auto || (pl->zmode != 0 && pl->zmode != 3) || pl->zfft_rows != 0 ||
         pl->thomas_async != -1 || pl->z_stages != 0 || pl->z_planes != 0)
         return;
     if (pl->sms <= 0 || !zline_supported(pl)) return;

@@ -393,24 +393,29 @@ cudaError_t launch_slab_n(const ZSlabArgs& a, const CUtensorMap& tm, int C, size
 static int slab_planes(const prj_plan* pl) {
     const Geometry& g = pl->g;
     const size_t most = (size_t)220 * 1024;
+    auto one_wave = [&](int H) {
+        const int C = (g.ny + H - 1) / H;
+        if (C > 8 || H > 256) return false;  // 256 planes: a tensor-map box
+        const size_t smem = slab_smem(g.nz, H) + 1024;  // the system's share of a CTA
+        if (smem > most) return false;
+        const int per_sm = std::min((int)((size_t)228 * 1024 / smem), 2);  // two by registers
+        return (long long)g.nxh * C <= (long long)per_sm * pl->sms;
+    };
     if (pl->z_planes > 0) {
+        // chunks of the kernel that z_mode 1 or 3 runs by default; else planes per CTA here
         const int H = std::min(pl->z_planes, g.ny);
-        return (g.ny + H - 1) / H <= 8 && slab_smem(g.nz, H) <= most ? H : 0;
+        return pl->zmode == 0 && one_wave(H) ? H : 0;
     }
     for (int C = 1; C <= 8 && C <= g.ny; C++) {
         const int H = (g.ny + C - 1) / C;
-        if (H > 256) continue;  // a tensor-map box
-        const size_t smem = slab_smem(g.nz, H) + 1024;  // the system's share of a CTA
-        if (smem > most) continue;
-        const int per_sm = std::min((int)((size_t)228 * 1024 / smem), 2);  // two by registers
-        if ((long long)g.nxh * ((g.ny + H - 1) / H) <= (long long)per_sm * pl->sms) return H;
+        if (one_wave(H)) return H;
     }
     return 0;
 }
 
 bool zslab_selected(const prj_plan* pl) {
     // a z kernel, row count, ring or stage count chosen by the plan's tuning stands
-    if (pl->zmode != pl->zmode_default || pl->zfft_rows != 0 || pl->thomas_async != -1 || pl->z_stages != 0) return false;
+    if (!pl->z_auto || pl->zfft_rows != 0 || pl->thomas_async != -1 || pl->z_stages != 0) return false;
     if (!pl->zd.ok || !pl->kz_of_slot || !pl->t.piv || !pl->spec || pl->g.nz > 1024) return false;
     return slab_planes(pl) > 0;
 }

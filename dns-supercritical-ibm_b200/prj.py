@@ -52,7 +52,7 @@ EXPORTS = (
     "prj_plan_enable_stage_timing", "prj_plan_stage_times", "prj_stage_name",
     "prj_poisson_fp64_noalloc", "prj_poisson_mixed",
     "prj_batch_create", "prj_batch_launch", "prj_batch_destroy", "prj_batch_info", "prj_batch_check_error",
-    "prj_plan_get_tuning", "prj_plan_set_tuning",
+    "prj_plan_get_tuning", "prj_plan_set_tuning", "prj_plan_set_z_auto", "prj_plan_get_z_auto",
     "prj_vd_metric_from_yu", "prj_plan_set_vd_metric", "prj_projection_step_vd",
     "prj_field_read_header", "prj_field_read", "prj_field_write", "prj_field_read_device",
     "prj_field_write_device", "prj_rough_force", "prj_ibm_interp", "prj_plan_schedule",
@@ -174,6 +174,8 @@ def load_library(path: str | None = None) -> ctypes.CDLL:
     L.prj_batch_check_error.argtypes = [_vp, _vp]
     L.prj_plan_get_tuning.argtypes = [_vp, ctypes.POINTER(Tuning)]
     L.prj_plan_set_tuning.argtypes = [_vp, ctypes.POINTER(Tuning)]
+    L.prj_plan_set_z_auto.argtypes = [_vp, ctypes.c_int]
+    L.prj_plan_get_z_auto.argtypes = [_vp, ctypes.POINTER(ctypes.c_int)]
     L.prj_vd_metric_from_yu.argtypes = [i, _dp, _dp]
     L.prj_plan_schedule.argtypes = [_vp, i, ctypes.POINTER(i)]
     L.prj_projection_step_host_async.argtypes = [_vp, _dp, _dp, _dp, _dp, _dp, _dp, _dp, ctypes.POINTER(StepParams), i]
@@ -427,20 +429,28 @@ class Plan:
     @property
     def tuning(self) -> dict:
         t = Tuning()
+        auto = ctypes.c_int()
         _check(load_library().prj_plan_get_tuning(self.handle, ctypes.byref(t)))
-        return t.as_dict()
+        _check(load_library().prj_plan_get_z_auto(self.handle, ctypes.byref(auto)))
+        return {**t.as_dict(), "z_auto": bool(auto.value)}
 
     def set_tuning(self, x_rows=None, z_rows=None, z_mode=None, **kw):
         """Change some fields of the plan's tuning (prj_plan_set_tuning); the others keep their
         current values.  Fields: x_rows, z_rows, z_mode, z_planes, z_stages, thomas_ring,
-        mixed_iters, mixed_tau, x_order, z_order."""
+        mixed_iters, mixed_tau, x_order, z_order; z_auto: the z kernels are picked by size
+        (prj_plan_set_z_auto), as on a new plan.  A z_mode without z_auto names the kernels."""
         t = self.tuning
+        if z_mode is not None:
+            t["z_auto"] = False
         for k, v in (("x_rows", x_rows), ("z_rows", z_rows), ("z_mode", z_mode), *kw.items()):
             if k not in t:
                 raise TypeError(f"unknown tuning field {k!r}")
             if v is not None:
                 t[k] = v
+        auto = t.pop("z_auto")
         _check(load_library().prj_plan_set_tuning(self.handle, ctypes.byref(Tuning(**t))))
+        if auto:
+            _check(load_library().prj_plan_set_z_auto(self.handle, 1))
 
     # ---------------------------------------------------------------- solve
     def poisson_mixed(self, P, stream=None):

@@ -313,11 +313,14 @@ int prj_batch_destroy(prj_batch* batch);
  *               3 = one kernel per x wavenumber on the compile-time pass plans (the
  *               three kernels where nz has no pass plan).  The default is 3 when
  *               nx/2+1 >= 2 x the SM count, else 0 (1 for nz with a prime factor above 5).
- *               With this and the next knobs at their defaults the plan picks by size:
- *               a whole x wavenumber on chip, one kernel per x wavenumber by one CTA or a
- *               cluster of them, or the three kernels (nz of any factors); the same bits;
- *   z_planes    planes per chunk of the per-wavenumber z kernels, planes per CTA of the
- *               on-chip one (0 = default);
+ *               A new plan picks its z kernels by size instead, while z_rows, z_stages and
+ *               thomas_ring are at their defaults (prj_plan_set_z_auto): a whole x wavenumber
+ *               on chip, one kernel per x wavenumber by one CTA or a cluster of them, or the
+ *               three kernels (nz of any factors); the same bits.  prj_plan_set_tuning names
+ *               the kernels: from then on the plan runs those of z_mode;
+ *   z_planes    planes per chunk of the per-wavenumber z kernels (0 = default); where the
+ *               plan picks by size and the default z_mode is 0, planes per CTA of the on-chip
+ *               kernel, if all its CTAs are then resident at once;
  *   z_stages    stages of their copy rings (0 = default, else 2..4; 2..8 for mode 1);
  *   thomas_ring shared-memory ring of the split Thomas kernel: -1 = default (none),
  *               0 = none, 1..4 = shapes 4x4, 8x2, 2x8, 8x3
@@ -350,6 +353,10 @@ typedef struct prj_tuning {
 } prj_tuning;
 int prj_plan_get_tuning(const prj_plan* plan, prj_tuning* out);
 int prj_plan_set_tuning(prj_plan* plan, const prj_tuning* tuning);
+/* on != 0: the plan picks its z kernels by size (again; z_mode returns to its default);
+ * 0: those of z_mode.  prj_plan_get_z_auto: which of the two. */
+int prj_plan_set_z_auto(prj_plan* plan, int on);
+int prj_plan_get_z_auto(const prj_plan* plan, int* on);
 
 /* Diagnostic of the bounded device-side waits of the pipelined kernels: one
  * kernel waits, for at most budget_cycles SM clock cycles, on an mbarrier that

@@ -132,3 +132,48 @@ def test_refused_lengths_stay_refused(cuda_device):
                 assert plan.tuning["z_mode"] == 1
                 with pytest.raises(prj.PrjError):
                     plan.set_tuning(z_mode=0)
+
+
+def test_z_mode_names_the_kernels(cuda_device):
+    """A z_mode that the caller gives is what runs, also where it is the plan's default; without
+    one, other fields and a round trip through the plan's tuning keep the choice by size."""
+    import prj
+    nx, ny, nz = 48, 33, 24
+    rhs = _rhs(nx, ny, nz, 5)
+    with _plan(nx, ny, nz) as plan:
+        t0 = plan.tuning
+        assert t0["z_mode"] == 0 and t0["z_auto"] and plan.launches_per_step() == 4
+        got = {"auto": _solve(plan, rhs)}
+        plan.set_tuning(z_mode=0)
+        assert plan.launches_per_step() == 6
+        got["split"] = _solve(plan, rhs)
+        plan.set_tuning(x_rows=4)
+        assert plan.launches_per_step() == 6
+        plan.set_tuning(**t0)
+        assert plan.tuning == t0 and plan.launches_per_step() == 4
+        plan.set_tuning(x_rows=4)
+        assert plan.tuning["z_auto"] and plan.launches_per_step() == 4
+        # the ABI: a tuning that was read and written back names the kernels it holds
+        import ctypes
+        t = prj.Tuning()
+        lib = prj.load_library()
+        assert lib.prj_plan_get_tuning(plan.handle, ctypes.byref(t)) == prj.PRJ_OK
+        assert lib.prj_plan_set_tuning(plan.handle, ctypes.byref(t)) == prj.PRJ_OK
+        assert plan.launches_per_step() == 6
+        assert lib.prj_plan_set_z_auto(plan.handle, 1) == prj.PRJ_OK
+        assert plan.launches_per_step() == 4
+    np.testing.assert_array_equal(got["auto"], got["split"])
+    with _plan(28, 9, 77) as plan:  # no in-place default: the fused kernel when named
+        assert plan.tuning["z_mode"] == 1
+        before = plan.launches_per_step()
+        plan.set_tuning(z_planes=4)
+        assert plan.launches_per_step() == 4
+        plan.set_tuning(z_planes=0, z_mode=1)
+        assert plan.launches_per_step() == 4 and not plan.tuning["z_auto"]
+        plan.set_tuning(z_auto=True)
+        assert plan.launches_per_step() == before
+    # planes per CTA that would take more than one wave of clusters
+    with _plan(400, 64, 64) as plan:
+        assert plan.tuning["z_mode"] == 0
+        plan.set_tuning(z_planes=8)
+        assert plan.launches_per_step() == 6
