@@ -48,4 +48,31 @@ inline cudaError_t launch_chained(bool chained, void (*kernel)(P...), dim3 grid,
     return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
+// Clusters of C CTAs along x that the device holds at once (a cluster's CTAs share one GPC, so
+// this is less than the free CTA slots divided by C: 15 clusters of 8 at one CTA per SM of 148).
+// 0 when the query fails.  Kernels asked about here are launched with the limit set here, the
+// device's: one value for all callers, so a thread that creates a plan takes nothing from one
+// that launches.
+constexpr int kSmemLimit = 227 * 1024;
+template <typename K>
+inline int resident_clusters(K kernel, unsigned threads, size_t smem, unsigned C) {
+    int most = 0;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(C);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = C;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&most, kernel, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return most;
+}
+
 }  // namespace prj

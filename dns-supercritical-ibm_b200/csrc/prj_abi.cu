@@ -447,15 +447,18 @@ bool split_z(const prj_plan* pl) {
 
 // z transforms + Thomas: three kernels (split) or one fused kernel
 int run_zsolve(prj_plan* pl, cudaStream_t st) {
-    if (prj::zslab_selected(pl)) {
+    if (pl->slab_h > 0) {
         StageTimer tm(pl, prj::kStZSolve, st);
         CK(prj::launch_zslab(pl, st), "z transform + Thomas (wavenumber on chip)");
         return PRJ_OK;
     }
-    if (prj::zline_cluster_selected(pl)) {
+    if (pl->zcl_c > 0) {
         StageTimer tm(pl, prj::kStZSolve, st);
-        CK(prj::launch_zline_cluster(pl, st), "z transform + Thomas (cluster per wavenumber)");
-        return PRJ_OK;
+        const cudaError_t e = prj::launch_zline_cluster(pl, st);
+        if (e != cudaErrorNotSupported) {
+            CK(e, "z transform + Thomas (cluster per wavenumber)");
+            return PRJ_OK;
+        }
     }
     if (pl->zmode == 3) {
         StageTimer tm(pl, prj::kStZSolve, st);
@@ -757,6 +760,7 @@ int prj_plan_create(int nx, int nz, int ny, double dx, double dz, const double* 
                          "Thomas pivots |D| in [%g, %g] leave the range [2^-40, 2^1000] of the forward sweeps' "
                          "correctly rounded division (a nearly singular wall-normal operator)",
                          mp, mm[1]));
+    prj::pick_z_route(pl);
     pl->device_bytes = bytes;
     *out = pl;
     return PRJ_OK;
@@ -1167,7 +1171,7 @@ bool x_pass_active(const prj_plan* pl) { return pl->use_pass && pl->fx64.even &&
 int prj_plan_schedule(const prj_plan* plan, int mode, int* launches) {
     if (!plan || !launches) return fail(PRJ_ERR_ARG, "NULL argument");
     if (mode == PRJ_MODE_FP64) {
-        const bool one_z = prj::zslab_selected(plan) || prj::zline_cluster_selected(plan) || !split_z(plan) || (plan->zmode == 3 && prj::zline_supported(plan));
+        const bool one_z = plan->slab_h > 0 || plan->zcl_c > 0 || !split_z(plan) || (plan->zmode == 3 && prj::zline_supported(plan));
         *launches = one_z ? 4 : 6;
     } else {
         // forward x, z transforms of the FP64 and FP32 rows, one Thomas launch, inverse z of both,
@@ -1185,6 +1189,8 @@ int prj_plan_set_z_auto(prj_plan* plan, int on) {
     if (rc) return rc;
     plan->z_auto = on != 0;
     if (on) plan->zmode = plan->zmode_default;
+    DeviceGuard dg(plan->device);
+    prj::pick_z_route(plan);
     return PRJ_OK;
 }
 
@@ -1291,6 +1297,7 @@ int prj_plan_set_tuning(prj_plan* plan, const prj_tuning* t) {
     plan->thomas_async = t->thomas_ring;
     plan->mixed_iters = t->mixed_iters;
     plan->mixed_tau = t->mixed_tau;
+    prj::pick_z_route(plan);
     return PRJ_OK;
 }
 

@@ -127,6 +127,8 @@ struct prj_plan {
     bool z_auto = true;           // the z kernels are picked by size (zmode is zmode_default); false
                                   // once a tuning names them
     int sms = 0;                  // SMs of the plan's device
+    int slab_h = 0;               // pick_z_route's choice: planes per CTA of the on-chip kernel (0: not it),
+    int zcl_c = 0, zcl_yb = 0;    // CTAs per wavenumber (0: not it; 1: k_zline) and planes per chunk
     bool use_pass = true;         // compile-time pass-plan FFT kernels where the length has one
     int thomas_async = -1;        // Thomas lines streamed through a cp.async shared-memory ring:
                                   // -1 and 0 never, 1..4 always (ring shape)
@@ -177,17 +179,24 @@ cudaError_t launch_stats(const prj_plan* pl, const double* U, const double* V, c
 // when the grid does not fit its shared-memory budget.  *err_word is raised if a
 // bounded wait gives up.
 cudaError_t launch_zsolve_pipelined(const prj_plan* pl, int* err_word, cudaStream_t st);
+int zslab_planes(const prj_plan* pl);                                   // prj_zslab.cu
+void zline_cluster_shape(const prj_plan* pl, int* C_out, int* yb_out);  // prj_zline.cu
 // z transform + Thomas + inverse z as one kernel per x wavenumber on the pass-plan
 // butterflies (prj_zline.cu); cudaErrorNotSupported when nz has no pass plan
 cudaError_t launch_zline(const prj_plan* pl, cudaStream_t st);
-// the same with a whole x wavenumber on chip, one cluster per wavenumber (prj_zslab.cu), where
-// the plan's z tuning is the default and the wavenumber fits; else cudaErrorNotSupported
+// the same with a whole x wavenumber on chip, one cluster per wavenumber (prj_zslab.cu);
+// cudaErrorNotSupported unless pick_z_route chose it
 cudaError_t launch_zslab(const prj_plan* pl, cudaStream_t st);
-bool zslab_selected(const prj_plan* pl);  // launch_zslab would run
-// the same as launch_zline with a cluster of CTAs per wavenumber (prj_zline.cu), or by it, where the
-// plan's z tuning is the default and its rule says so
+// the same as launch_zline with a cluster of CTAs per wavenumber (prj_zline.cu), or by it;
+// cudaErrorNotSupported unless pick_z_route chose it, or when the driver refuses the tensor map
 cudaError_t launch_zline_cluster(const prj_plan* pl, cudaStream_t st);
-bool zline_cluster_selected(const prj_plan* pl);  // launch_zline_cluster would run
+// which of the two runs (slab_h, zcl_c, zcl_yb) by the rules beside them, where the plan's z
+// tuning is the default; once per plan and per change of its tuning, on the plan's device
+inline void pick_z_route(prj_plan* pl) {
+    pl->zcl_c = pl->zcl_yb = 0;
+    pl->slab_h = zslab_planes(pl);
+    if (pl->slab_h == 0) zline_cluster_shape(pl, &pl->zcl_c, &pl->zcl_yb);
+}
 bool zline_supported(const prj_plan* pl);  // launch_zline would run (not fall back)
 
 // x transforms with the in-place DIF FFT (prj_xfft.cu); used when pl->xd.ok

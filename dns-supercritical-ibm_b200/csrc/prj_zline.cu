@@ -47,15 +47,6 @@ __global__ void __launch_bounds__(zl_threads(PL::n, zl_lpt(PL::n)), zl_minb(zl_t
 }
 
 template <class PL>
-cudaError_t launch_zline_cluster_pl(const ZLineArgs& a, const CUtensorMap& tm, size_t smem, cudaStream_t st) {
-    cudaError_t e =
-        cudaFuncSetAttribute(k_zline_cluster<PL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    return launch_chained(false, k_zline_cluster<PL>, dim3((unsigned)(a.nh * a.C)), zl_threads(PL::n, zl_lpt(PL::n)), smem, st,
-                          (unsigned)a.C, a, tm);
-}
-
-template <class PL>
 cudaError_t launch_zline_ns(const ZLineArgs& a, const CUtensorMap& tm, int ns, size_t smem, cudaStream_t st) {
     constexpr int L = zl_lpt(PL::n);
     switch (ns) {
@@ -126,56 +117,73 @@ bool zline_tmap(void* tmap128, const double2* X, int n, int nh, int ny, int yb) 
     return tmap_encode_f64(tmap128, X, 4, dims, strides, box);
 }
 
+// the cluster kernel of the plan's z length, null for the lengths that its rule leaves out
+using ZClusterKernel = void (*)(ZLineArgs, CUtensorMap);
+constexpr int kZClusterMaxN = 384;
+template <class PL>
+static ZClusterKernel zcluster_kernel_of() {
+    if constexpr (PL::n <= kZClusterMaxN) return k_zline_cluster<PL>;
+    else return nullptr;
+}
+static ZClusterKernel zcluster_kernel(const prj_plan* pl) {
+#define PRJ_ZL_CASE(N, ...) \
+    if (pl->g.nz == N && same_radices<PassList<__VA_ARGS__>>(pl->zd.f)) return zcluster_kernel_of<PassList<__VA_ARGS__>>();
+    PRJ_PASS_ALL(PRJ_ZL_CASE)
+#undef PRJ_ZL_CASE
+    return nullptr;
+}
+
 // CTAs per wavenumber C and planes per chunk of the cluster form; C = 0 where it does not apply.
-// The most CTAs (up to 8) that are all resident at once: a second wave would double the chain.
-// C = 1 (k_zline) where there is a wavenumber per SM at least.  Measured (z solve, us, by cluster
-// / one CTA / three kernels): 58 / 74 / 83 at 256 x 128 x 128 (C = 3), 150 / 169 / 210 at
-// 384 x 192 x 192 (C = 2), 65 / 89 / 96 at 384 x 138 x 96, 50 / 56 / 58 at 192 x 42 x 384; - / 308 /
-// 398 at 512 x 256 x 256; but 132 / 198 / 92 at 64 x 130 x 512 and 107 / 222 / 60 at 64 x 53 x 768,
-// whose few wavenumbers have long rows (nz above 384 is left to the three kernels).
-static void zline_cluster_shape(const prj_plan* pl, int* C_out, int* yb_out) {
+// The most CTAs, up to 4, whose clusters are all resident at once (as the runtime answers): a
+// second wave would double the chain.  Measured (Poisson solve, us, by cluster / one CTA / three
+// kernels): 102 / 118 / 124 at 256 x 128 x 128 (C = 3), 306 / 323 / 366 at 384 x 192 x 192 (C = 2),
+// 212 / 287 / 244 at 96 x 300 x 256 and 79 / 150 / 79 at 48 x 105 x 384 (C = 4; 322 and 96 with 8, the
+// first in two waves), 203 / 426 / 246 at 64 x 300 x 384 (238 with 8).  Lengths above 384 gain
+// little or lose: 82 / 119 / 72 at 64 x 64 x 512, 598 / 1032 / 544 at 96 x 292 x 768.
+// C = 1 (k_zline) below two wavenumbers per SM, from where z_mode's default takes it: with a
+// wavenumber per SM up to nz = 384 and 1.25 up to 768 (one CTA / three kernels): 517 / 524 at
+// 350 x 100 x 512 and 1054 / 1106 at 400 x 128 x 768, but 933 / 886 at 300 x 200 x 512, 938 / 855 at
+// 300 x 128 x 768, and with four and eight lines per thread 1234 / 1082 at 400 x 100 x 1024, 1061 /
+// 830 at 300 x 60 x 1536.
+void zline_cluster_shape(const prj_plan* pl, int* C_out, int* yb_out) {
     *C_out = *yb_out = 0;
     const Geometry& g = pl->g;
     // a z kernel, row count, ring, chunk or stage count chosen by the plan's tuning stands
-    if (!pl->z_auto || (pl->zmode != 0 && pl->zmode != 3) || pl->zfft_rows != 0 ||
-        pl->thomas_async != -1 || pl->z_stages != 0 || pl->z_planes != 0)
+    if (!pl->z_auto || (pl->zmode != 0 && pl->zmode != 3) || pl->zfft_rows != 0 || pl->thomas_async != -1 ||
+        pl->z_stages != 0 || pl->z_planes != 0)
         return;
     if (pl->sms <= 0 || !zline_supported(pl)) return;
-    const int nt = zl_threads(g.nz, zl_lpt(g.nz));
-    for (int C = g.nz <= 384 ? 8 : 1; C >= 2; C--) {
+    const unsigned nt = (unsigned)zl_threads(g.nz, zl_lpt(g.nz));
+    const ZClusterKernel kernel = zcluster_kernel(pl);
+    for (int C = kernel ? 4 : 1; C >= 2; C--) {
         const int per_sm = (g.nxh * C + pl->sms - 1) / pl->sms;
-        if (per_sm > zl_minb(nt)) continue;
+        if (per_sm > zl_minb((int)nt)) continue;
         const size_t most = (size_t)228 * 1024 / per_sm - 1024;
         int yb = 8;
         while (yb > 1 && zline_cluster_smem(g.nz, g.mzp, yb, 2) > std::min(most, (size_t)220 * 1024)) yb--;
         if (yb < 2 || yb * C > g.ny) continue;
+        if (resident_clusters(kernel, nt, zline_cluster_smem(g.nz, g.mzp, yb, 2), (unsigned)C) < g.nxh) continue;
         *C_out = C;
         *yb_out = yb;
         return;
     }
-    if (g.nxh >= pl->sms) *C_out = 1;
-}
-
-bool zline_cluster_selected(const prj_plan* pl) {
-    int C, yb;
-    zline_cluster_shape(pl, &C, &yb);
-    return C > 0;
+    if (g.nz <= 384 ? g.nxh >= pl->sms : g.nz <= 768 && 4 * g.nxh >= 5 * pl->sms) *C_out = 1;
 }
 
 cudaError_t launch_zline_cluster(const prj_plan* pl, cudaStream_t st) {
     const Geometry& g = pl->g;
+    if (pl->zcl_c == 1) return launch_zline(pl, st);
+    const ZClusterKernel kernel = zcluster_kernel(pl);
     ZLineArgs a = zline_args(pl);
-    zline_cluster_shape(pl, &a.C, &a.yb);
-    if (a.C == 1) return launch_zline(pl, st);
+    a.C = pl->zcl_c;
+    a.yb = pl->zcl_yb;
     CUtensorMap tm{};
-    if (a.C < 2 || !zline_tmap(&tm, pl->spec, g.nz, g.nxh, g.ny, a.yb)) return cudaErrorInvalidValue;
+    if (a.C < 2 || !kernel || !zline_tmap(&tm, pl->spec, g.nz, g.nxh, g.ny, a.yb)) return cudaErrorNotSupported;
     const size_t smem = zline_cluster_smem(g.nz, g.mzp, a.yb, 2);
-#define PRJ_ZL_CASE(N, ...)                                                  \
-    if (g.nz == N && same_radices<PassList<__VA_ARGS__>>(pl->zd.f))          \
-        return launch_zline_cluster_pl<PassList<__VA_ARGS__>>(a, tm, smem, st);
-    PRJ_PASS_ALL(PRJ_ZL_CASE)
-#undef PRJ_ZL_CASE
-    return cudaErrorInvalidValue;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
+    if (e != cudaSuccess) return e;
+    return launch_chained(false, kernel, dim3((unsigned)(a.nh * a.C)), (unsigned)zl_threads(g.nz, zl_lpt(g.nz)), smem, st,
+                          (unsigned)a.C, a, tm);
 }
 
 // cudaErrorNotSupported when nz has no pass plan (the caller runs the split kernels)

@@ -367,39 +367,50 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_zslab(const __grid_constant__ 
     }
 }
 
-template <class FFT, int NT, int LPT>
-cudaError_t launch_slab(const ZSlabArgs& a, const CUtensorMap& tm, int C, size_t smem, bool chained, cudaStream_t st) {
-    auto kernel = k_zslab<FFT, NT, LPT>;
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    return launch_chained(chained, kernel, dim3((unsigned)C, (unsigned)a.nh), NT, smem, st, (unsigned)C, a, tm);
-}
+using SlabKernel = void (*)(ZSlabArgs, CUtensorMap);
+constexpr int kSlabThreads = 256;
+constexpr int kSlabMaxN = 512;
 
 template <class FFT, int N>
-cudaError_t launch_slab_n(const ZSlabArgs& a, const CUtensorMap& tm, int C, size_t smem, bool chained,
-                          cudaStream_t st) {
-    constexpr int NT = 256, LPT = (N + NT - 1) / NT;
-    return launch_slab<FFT, NT, LPT>(a, tm, C, smem, chained, st);
+SlabKernel slab_kernel_n() {
+    if constexpr (N <= kSlabMaxN) return k_zslab<FFT, kSlabThreads, (N + kSlabThreads - 1) / kSlabThreads>;
+    else return nullptr;
+}
+
+// the kernel of the plan's z length (nz <= kSlabMaxN), by the radix order in use
+SlabKernel slab_kernel(const prj_plan* pl) {
+    const int nz = pl->g.nz;
+#define PRJ_SLAB_CASE(N, ...)                                          \
+    if (nz == N && same_radices<PassList<__VA_ARGS__>>(pl->zd.f))      \
+        return slab_kernel_n<PassFft<PassList<__VA_ARGS__>>, N>();
+    PRJ_PASS_ALL(PRJ_SLAB_CASE)
+#undef PRJ_SLAB_CASE
+    return nz <= 256 ? k_zslab<RuntimeFft, kSlabThreads, 1> : k_zslab<RuntimeFft, kSlabThreads, 2>;
 }
 
 }  // namespace
 
 // planes per CTA of the slab kernel, 0 where it does not apply: the plan's z_planes tuning, or
-// the fewest CTAs per wavenumber (at most 8) with which every cluster is resident at once.  The
-// kernel is one dependent pass over the planes, so a second wave of clusters doubles its time:
-// measured (z solve, us, slab / three kernels), 13 / 28 at 48 x 32 x 24, 25 / 45 at
-// 128 x 96 x 64, 27 / 41 at 512 x 55 x 64, 97 / 107 at 64 x 324 x 80, each in one wave, but
-// 78 / 73 at 256 x 128 x 128 and 133 / 90 at 768 x 213 x 32 in two or three.
-static int slab_planes(const prj_plan* pl) {
+// the fewest CTAs per wavenumber (at most 8) with which every cluster is resident at once, up to
+// nz = 512.  The kernel is one dependent pass over the planes, so a second wave of clusters doubles
+// its time, and how many are resident is asked of the runtime.  Measured (Poisson solve, us, slab
+// / three kernels), 20 / 29 at 48 x 32 x 24, 37 / 51 at 128 x 96 x 64, 49 / 59 at 512 x 55 x 64, 78 /
+// 118 at 64 x 324 x 80, each in one wave, but 119 / 124 at 256 x 128 x 128, 155 / 123 at 32 x 256 x
+// 224 and 134 / 73 at 32 x 68 x 768 in more.  With three lines per thread and more the chain
+// loses in one wave too: 87 / 64 at 32 x 64 x 640, 68 / 50 at 32 x 32 x 1000; 44 / 46 at 64 x 32 x 512.
+int zslab_planes(const prj_plan* pl) {
     const Geometry& g = pl->g;
-    const size_t most = (size_t)220 * 1024;
+    // z kernels, a row count, a ring or a stage count chosen by the plan's tuning stand
+    if (!pl->z_auto || pl->zfft_rows != 0 || pl->thomas_async != -1 || pl->z_stages != 0) return 0;
+    if (!pl->zd.ok || !pl->kz_of_slot || !pl->t.piv || !pl->spec || g.nz > kSlabMaxN) return 0;
+    const SlabKernel kernel = slab_kernel(pl);
     auto one_wave = [&](int H) {
         const int C = (g.ny + H - 1) / H;
         if (C > 8 || H > 256) return false;  // 256 planes: a tensor-map box
-        const size_t smem = slab_smem(g.nz, H) + 1024;  // the system's share of a CTA
-        if (smem > most) return false;
-        const int per_sm = std::min((int)((size_t)228 * 1024 / smem), 2);  // two by registers
-        return (long long)g.nxh * C <= (long long)per_sm * pl->sms;
+        const size_t smem = slab_smem(g.nz, H);
+        if (smem + 1024 > (size_t)220 * 1024) return false;
+        // two CTAs per SM by registers: no need to ask for what cannot fit
+        return (long long)g.nxh * C <= 2LL * pl->sms && resident_clusters(kernel, kSlabThreads, smem, (unsigned)C) >= g.nxh;
     };
     if (pl->z_planes > 0) {
         // chunks of the kernel that z_mode 1 or 3 runs by default; else planes per CTA here
@@ -413,16 +424,10 @@ static int slab_planes(const prj_plan* pl) {
     return 0;
 }
 
-bool zslab_selected(const prj_plan* pl) {
-    // a z kernel, row count, ring or stage count chosen by the plan's tuning stands
-    if (!pl->z_auto || pl->zfft_rows != 0 || pl->thomas_async != -1 || pl->z_stages != 0) return false;
-    if (!pl->zd.ok || !pl->kz_of_slot || !pl->t.piv || !pl->spec || pl->g.nz > 1024) return false;
-    return slab_planes(pl) > 0;
-}
-
 cudaError_t launch_zslab(const prj_plan* pl, cudaStream_t st) {
     const Geometry& g = pl->g;
-    const int H = slab_planes(pl);
+    const int H = pl->slab_h;
+    if (H <= 0) return cudaErrorNotSupported;
     ZSlabArgs a{};
     a.n = g.nz; a.ny = g.ny; a.nh = g.nxh; a.nzh = g.nzh; a.nzhdiv = make_fastdiv((unsigned)g.nzh); a.mzp = g.mzp;
     a.rs = (g.nz + 7) & ~7; a.H = H; a.hp = slab_pitch(H);
@@ -431,18 +436,12 @@ cudaError_t launch_zslab(const prj_plan* pl, cudaStream_t st) {
     a.err = reinterpret_cast<int*>(pl->stat_buf + kStatErrSlot);
     CUtensorMap tm{};
     a.tma = zline_tmap(&tm, pl->spec, g.nz, g.nxh, g.ny, H) ? 1 : 0;
-    const int C = (g.ny + H - 1) / H;
+    const unsigned C = (unsigned)((g.ny + H - 1) / H);
     const size_t smem = slab_smem(g.nz, H);
-    const bool ch = chained(pl);
-#define PRJ_SLAB_CASE(N, ...)                                                            \
-    if (g.nz == N && same_radices<PassList<__VA_ARGS__>>(pl->zd.f))                      \
-        return launch_slab_n<PassFft<PassList<__VA_ARGS__>>, N>(a, tm, C, smem, ch, st);
-    PRJ_PASS_ALL(PRJ_SLAB_CASE)
-#undef PRJ_SLAB_CASE
-    if (g.nz <= 256) return launch_slab<RuntimeFft, 256, 1>(a, tm, C, smem, ch, st);
-    if (g.nz <= 512) return launch_slab<RuntimeFft, 256, 2>(a, tm, C, smem, ch, st);
-    if (g.nz <= 1024) return launch_slab<RuntimeFft, 256, 4>(a, tm, C, smem, ch, st);
-    return cudaErrorNotSupported;
+    const SlabKernel kernel = slab_kernel(pl);
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
+    if (e != cudaSuccess) return e;
+    return launch_chained(chained(pl), kernel, dim3(C, (unsigned)g.nxh), kSlabThreads, smem, st, C, a, tm);
 }
 
 }  // namespace prj

@@ -177,3 +177,17 @@ def test_z_mode_names_the_kernels(cuda_device):
         assert plan.tuning["z_mode"] == 0
         plan.set_tuning(z_planes=8)
         assert plan.launches_per_step() == 6
+
+
+# wavenumbers x CTAs that free SM slots would hold but the GPCs do not, long rows on chip, and
+# k_zline below two wavenumbers per SM at long rows, each slower than the three kernels; clusters of
+# four where more would also be resident
+@pytest.mark.parametrize("shape,launches", [((32, 68, 768), 6), ((32, 256, 240), 6), ((32, 384, 160), 6),
+                                            ((36, 83, 600), 6), ((32, 64, 640), 6), ((300, 24, 1536), 6),
+                                            ((300, 100, 1024), 6), ((96, 300, 256), 4), ((48, 105, 384), 4),
+                                            ((32, 400, 384), 4)])
+def test_routes_where_a_second_wave_would_run(cuda_device, shape, launches):
+    nx, ny, nz = shape
+    got, want, n = _both(nx, ny, nz, _rhs(nx, ny, nz, 6))
+    assert n == launches
+    np.testing.assert_array_equal(got, want)
