@@ -687,7 +687,7 @@ int prj_plan_create(int nx, int nz, int ny, double dx, double dz, const double* 
     pl->thomas_async = -1;
     pl->kxs = g.nxh;
     pl->tz_xd = prj::choose_tz_xd(pl->fx64.m, pl->fx64.even);
-    pl->tz_xp = prj::choose_tz_xp(pl->fx64.m);
+    pl->tz_xp = prj::choose_tz_xp(pl->fx64.m, (long long)nz * ny);
 
     // rows per CTA of the x kernels: fit two ping-pong buffers in ~100 KB
     {

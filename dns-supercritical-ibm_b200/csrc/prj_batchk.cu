@@ -259,10 +259,12 @@ cudaError_t batchk_build(prj_plan* const* plans, double* const* d_P, int ncases,
         c.x = batch_x_args(pl, d_P[i]);
         c.zl = zline_args(pl);
         // x tile shapes within the per-case kernels' default shared-memory budgets and, with
-        // their staged input, within kStagedBytes, so six CTAs fit per SM whatever the
-        // plans' own tuning; a tile's shape does not change its results
+        // their staged input, within kStagedBytes, so six CTAs fit per SM: as many rows
+        // as fit, or x_rows where the plan's tuning asks for fewer (its default count stands for no
+        // request, as a tuning that was read and written back holds it); a tile's shape does not
+        // change its results
         const int m = pl->fx64.m;
-        c.x.tz = c.x.tz == choose_tz_xp(m) ? fit_tz_xp(m) : std::min(c.x.tz, fit_tz_xp(m));
+        c.x.tz = c.x.tz == choose_tz_xp(m, (long long)g.nz * g.ny) ? fit_tz_xp(m) : std::min(c.x.tz, fit_tz_xp(m));
         while (c.x.tz > 1 && pass_x_smem(m, c.x.tz) + x_stage_bytes(m, c.x.tz) > kStagedBytes) c.x.tz /= 2;
         c.soff = (int)pass_x_smem(m, c.x.tz);
         c.xboxes = x_boxes(m);

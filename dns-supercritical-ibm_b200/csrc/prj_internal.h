@@ -215,7 +215,7 @@ inline cudaError_t launch_fwd_x_range(const prj_plan* pl, const double* Uh, cons
     return launch_fwd_xd(pl, FwdSource::Divergence, nullptr, Uh, Vh, Wh, sc, st, nullptr, yr);
 }
 int choose_tz_xd(int m, bool even);
-int choose_tz_xp(int m);                 // rows per CTA of the pass-plan x kernels
+int choose_tz_xp(int m, long long rows);  // rows per CTA of the tiled x kernels, a grid of `rows` x-rows
 int fit_tz_xp(int m);                    // the most rows per CTA that fit
 size_t pass_x_smem(int m, int tz);       // their shared memory
 
