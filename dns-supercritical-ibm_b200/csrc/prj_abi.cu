@@ -126,50 +126,41 @@ void dfree(P*& p) {
     p = nullptr;
 }
 
-// in-place DIF tables of a length-n transform in radix order `order` (left unset when a
-// radix is unsupported)
-int make_dif(int n, prj::DifFft* d, size_t* bytes, int order = 0) {
+// In-place DIF tables of a length-n transform in radix order `order` (`ok` stays false, and no
+// twiddles are made, when a prime factor is too large); with `slots` (the z axis) also the tables by
+// slot: the wavenumber of each slot (n, the inverse of the position table; natural order where the
+// out-of-place transforms leave that); the pair of each slot (n) and of each folded wavenumber
+// min(kz, n - kz) (n/2 + 1), the pairs numbered in the order of their first slots.  One
+// allocation and one copy for all of them: a plan's creation is mostly cudaMalloc and cudaFree.
+int make_dif(int n, prj::DifFft* d, size_t* bytes, int order = 0, int** slots = nullptr) {
     d->ok = false;
-    if (!prj::dif_supported(n)) return PRJ_OK;
-    const long ntw = prj::dif_plan(n, &d->f, order);
-    if (ntw < 0) return PRJ_OK;
-    std::vector<double2> tw((size_t)ntw);
-    std::vector<int> pos((size_t)n);
-    prj::dif_fill(d->f, tw.data(), pos.data());
-    CK(cudaMalloc((void**)&d->tw, tw.size() * sizeof(double2)), "cudaMalloc(DIF twiddles)");
-    CK(cudaMemcpy(d->tw, tw.data(), tw.size() * sizeof(double2), cudaMemcpyHostToDevice), "cudaMemcpy(DIF twiddles)");
-    CK(cudaMalloc((void**)&d->pos, pos.size() * sizeof(int)), "cudaMalloc(DIF positions)");
-    CK(cudaMemcpy(d->pos, pos.data(), pos.size() * sizeof(int), cudaMemcpyHostToDevice), "cudaMemcpy(DIF positions)");
-    *bytes += tw.size() * sizeof(double2) + pos.size() * sizeof(int);
-    d->ok = true;
-    return PRJ_OK;
-}
-
-// tables of the length-n in-place plan, one after the other: the wavenumber of each slot
-// (n, the inverse of the position table); the pair of each slot (n) and of each folded
-// wavenumber min(kz, n - kz) (n/2 + 1), the pairs numbered in the order of their first slots
-int slot_table_len(int n) { return 2 * n + n / 2 + 1; }
-int make_slot_table(int n, int** d_out, size_t* bytes, int order = 0) {
-    std::vector<int> pos((size_t)n), tab((size_t)slot_table_len(n), -1);
-    if (prj::dif_supported(n)) {
-        prj::DifDev f{};
-        const long ntw = prj::dif_plan(n, &f, order);
-        if (ntw < 0) return fail(PRJ_ERR_UNSUPPORTED, "no in-place plan for length %d", n);
-        std::vector<double2> tw((size_t)ntw);
-        prj::dif_fill(f, tw.data(), pos.data());
-    } else {  // the out-of-place transforms leave natural order
-        for (int k = 0; k < n; k++) pos[k] = k;
+    const long ntw = prj::dif_supported(n) ? prj::dif_plan(n, &d->f, order) : -1;
+    if (ntw < 0 && !slots) return PRJ_OK;
+    const size_t tw_bytes = ntw < 0 ? 0 : (size_t)ntw * sizeof(double2), npos = (size_t)n;
+    const size_t nslots = slots ? 2 * npos + npos / 2 + 1 : 0;
+    std::vector<unsigned char> host(tw_bytes + (npos + nslots) * sizeof(int));
+    int* pos = reinterpret_cast<int*>(host.data() + tw_bytes);
+    if (ntw >= 0) prj::dif_fill(d->f, reinterpret_cast<double2*>(host.data()), pos);
+    else for (int k = 0; k < n; k++) pos[k] = k;
+    if (slots) {
+        int* tab = pos + n;
+        std::fill(tab, tab + nslots, -1);
+        for (int k = 0; k < n; k++) tab[pos[k]] = k;
+        int next = 0;
+        for (int s = 0; s < n; s++) {
+            int& pair = tab[2 * n + std::min(tab[s], n - tab[s])];
+            if (pair < 0) pair = next++;
+            tab[n + s] = pair;
+        }
     }
-    for (int k = 0; k < n; k++) tab[pos[k]] = k;
-    int next = 0;
-    for (int s = 0; s < n; s++) {
-        int& pair = tab[2 * n + std::min(tab[s], n - tab[s])];
-        if (pair < 0) pair = next++;
-        tab[n + s] = pair;
-    }
-    CK(cudaMalloc((void**)d_out, tab.size() * sizeof(int)), "cudaMalloc(slot table)");
-    CK(cudaMemcpy(*d_out, tab.data(), tab.size() * sizeof(int), cudaMemcpyHostToDevice), "cudaMemcpy(slot table)");
-    *bytes += tab.size() * sizeof(int);
+    CK(cudaMalloc(&d->block, host.size()), "cudaMalloc(DIF tables)");
+    CK(cudaMemcpy(d->block, host.data(), host.size(), cudaMemcpyHostToDevice), "cudaMemcpy(DIF tables)");
+    d->bytes = host.size();
+    *bytes += d->bytes;
+    d->tw = static_cast<double2*>(d->block);
+    d->pos = reinterpret_cast<int*>(static_cast<unsigned char*>(d->block) + tw_bytes);
+    if (slots) *slots = d->pos + n;
+    d->ok = ntw >= 0;
     return PRJ_OK;
 }
 
@@ -192,11 +183,9 @@ void free_plan_buffers(prj_plan* pl) {
     dfree(pl->fx64.tw);
     dfree(pl->fx64.post);
     dfree(pl->fz64.tw);
-    dfree(pl->xd.tw);
-    dfree(pl->xd.pos);
-    dfree(pl->zd.tw);
-    dfree(pl->zd.pos);
-    dfree(pl->kz_of_slot);
+    dfree(pl->xd.block);
+    dfree(pl->zd.block);
+    pl->kz_of_slot = nullptr;
     dfree(pl->spec32);
     dfree(pl->pbar);
     dfree(pl->psum);
@@ -673,8 +662,7 @@ int prj_plan_create(int nx, int nz, int ny, double dx, double dz, const double* 
     if ((rc = make_rfft<double>(nx, &pl->fx64, &bytes))) return bail(rc);
     if ((rc = make_cfft<double>(nz, &pl->fz64.f, &pl->fz64.tw, &bytes))) return bail(rc);
     if ((rc = make_dif(pl->fx64.m, &pl->xd, &bytes))) return bail(rc);
-    if ((rc = make_dif(nz, &pl->zd, &bytes))) return bail(rc);
-    if ((rc = make_slot_table(nz, &pl->kz_of_slot, &bytes))) return bail(rc);
+    if ((rc = make_dif(nz, &pl->zd, &bytes, 0, &pl->kz_of_slot))) return bail(rc);
     {
         int sms = 0;
         if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, pl->device) != cudaSuccess) sms = 0;
@@ -1222,25 +1210,17 @@ int reorder_dif(prj_plan* pl, bool x_axis, int order) {
     prj::DifFft fresh{};
     size_t bytes = 0;
     int* kz = nullptr;
-    int rc = make_dif(n, &fresh, &bytes, order);
-    if (!rc && !x_axis && fresh.ok) rc = make_slot_table(n, &kz, &bytes, order);
+    const int rc = make_dif(n, &fresh, &bytes, order, x_axis ? nullptr : &kz);
     if (rc || !fresh.ok) {
-        dfree(fresh.tw);
-        dfree(fresh.pos);
-        dfree(kz);
+        dfree(fresh.block);
         return rc ? rc : fail(PRJ_ERR_UNSUPPORTED, "no in-place plan of length %d in radix order %d", n, order);
     }
     cudaDeviceSynchronize();
     prj::DifFft& d = x_axis ? pl->xd : pl->zd;
-    const size_t old = (size_t)prj::dif_twiddle_count(d.f) * sizeof(double2) + (size_t)n * sizeof(int) +
-                       (x_axis ? 0 : (size_t)slot_table_len(n) * sizeof(int));
-    dfree(d.tw);
-    dfree(d.pos);
+    const size_t old = d.bytes;
+    dfree(d.block);
     d = fresh;
-    if (!x_axis) {
-        dfree(pl->kz_of_slot);
-        pl->kz_of_slot = kz;
-    }
+    if (!x_axis) pl->kz_of_slot = kz;
     pl->device_bytes += bytes;
     pl->device_bytes -= std::min(old, pl->device_bytes);
     (x_axis ? pl->x_order : pl->z_order) = order;

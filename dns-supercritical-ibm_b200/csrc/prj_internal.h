@@ -24,6 +24,8 @@ struct DifFft {
     DifDev f{};
     double2* tw = nullptr;  // stage twiddles (forward sign)
     int* pos = nullptr;     // pos[k]: slot of index k after the transform
+    void* block = nullptr;  // the allocation that holds them (z: and kz_of_slot)
+    size_t bytes = 0;
 };
 
 // One real-to-complex transform of length n along a contiguous axis, done as a

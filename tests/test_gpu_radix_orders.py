@@ -79,3 +79,16 @@ def test_batch_with_other_orders(cuda_device):
             np.testing.assert_array_equal(from_dev(t), want)
     for p in plans:
         p.close()
+
+
+def test_device_bytes_follow_the_tables(cuda_device):
+    """The in-place tables of an axis are one allocation, replaced as a whole by another order."""
+    import prj
+    import workloads
+    _, yu, dx, dz = workloads.poisson_rhs(128, 21, 64, seed=1)
+    with prj.Plan(128, 64, 21, dx, dz, prj.bands(yu, "consistent")) as plan:
+        t0, before = plan.tuning, plan.device_bytes
+        plan.set_tuning(x_order=1, z_order=1)
+        assert plan.device_bytes > 0
+        plan.set_tuning(**t0)
+        assert plan.device_bytes == before
