@@ -30,7 +30,7 @@ __device__ __forceinline__ size_t hidx(int nx, int nz, int i, int j, int k) {
 
 struct FwdArgs {
     int nx, nz, ny, nh, m, tz, rs;
-    int even;
+    int even, pairs;  // pairs: P lies on a 16-byte boundary, its x pairs move as one access
     FftDev f;
     const double2* tw;
     const double2* post;
@@ -76,7 +76,8 @@ __global__ void __launch_bounds__(256) k_fwd_x(const FwdArgs a) {
         if (z < a.nz) {
             if (SRC == 0) {
                 const double* row = a.P + ((size_t)y * a.nz + z) * a.nx;
-                if (a.even) v = reinterpret_cast<const double2*>(row)[n];
+                if (a.even && a.pairs) v = reinterpret_cast<const double2*>(row)[n];
+                else if (a.even) v = make_double2(row[2 * n], row[2 * n + 1]);
                 else v.x = row[n];
             } else {
                 if (a.even) { v.x = divergence_at(a, 2 * n, z, y); v.y = divergence_at(a, 2 * n + 1, z, y); }
@@ -114,7 +115,7 @@ __global__ void __launch_bounds__(256) k_fwd_x(const FwdArgs a) {
 
 struct BwdArgs {
     int nx, nz, ny, nh, m, tz, rs;
-    int even;
+    int even, pairs;
     FftDev f;
     const double2* tw;
     const double2* post;
@@ -171,7 +172,8 @@ __global__ void __launch_bounds__(256) k_bwd_x(const BwdArgs a) {
         if (z >= a.nz) continue;
         double* row = a.P + ((size_t)y * a.nz + z) * a.nx;
         const double2 v = F[r * a.rs + n];
-        if (a.even) reinterpret_cast<double2*>(row)[n] = v;
+        if (a.even && a.pairs) reinterpret_cast<double2*>(row)[n] = v;
+        else if (a.even) row[2 * n] = v.x, row[2 * n + 1] = v.y;
         else row[n] = v.x;
     }
 }
@@ -444,6 +446,7 @@ cudaError_t launch_fwd_x(const prj_plan* pl, FwdSource src, const double* P, con
     a.m = pl->fx64.m; a.tz = pl->tz_fwd; a.rs = pl->fx64.m + 1; a.even = pl->fx64.even;
     a.f = pl->fx64.f; a.tw = pl->fx64.tw; a.post = pl->fx64.post;
     a.P = P; a.Uh = Uh; a.Vh = Vh; a.Wh = Wh; a.inv_dy_p = pl->t.inv_dy_p;
+    a.pairs = ((uintptr_t)P & 15u) == 0;
     a.inv_dx = 1.0 / g.dx; a.inv_dz = 1.0 / g.dz;
     if (sc) { a.inv_dt = sc->inv_dt; a.vbot = sc->wall[1]; a.vtop = sc->wall[4]; }
     a.X = pl->spec;
@@ -467,7 +470,7 @@ cudaError_t launch_bwd_x(const prj_plan* pl, double* P, cudaStream_t st) {
     a.nx = g.nx; a.nz = g.nz; a.ny = g.ny; a.nh = g.nxh;
     a.m = pl->fx64.m; a.tz = pl->tz_fwd; a.rs = pl->fx64.m + 1; a.even = pl->fx64.even;
     a.f = pl->fx64.f; a.tw = pl->fx64.tw; a.post = pl->fx64.post;
-    a.X = pl->spec; a.P = P;
+    a.X = pl->spec; a.P = P; a.pairs = ((uintptr_t)P & 15u) == 0;
     a.scale = 1.0 / ((double)g.nx * (double)g.nz + 0.0);
     const size_t smem = (size_t)2 * a.tz * a.rs * sizeof(double2);
     cudaError_t e = set_smem(k_bwd_x, smem);
