@@ -173,6 +173,8 @@ int prj_dist_thomas(prj_plan* plan, double* d_lines, int kx0, int kx1, void* str
     if (kx0 < 0 || kx1 > plan->g.nxh || kx0 > kx1) return record_error(PRJ_ERR_ARG, "prj_dist_thomas: bad x-wavenumber range");
     if (kx1 == kx0) return PRJ_OK;
     if (!d_lines) return record_error(PRJ_ERR_ARG, "prj_dist_thomas: line buffer is NULL");
+    if ((uintptr_t)d_lines & 15u)  // read as whole complex values
+        return record_error(PRJ_ERR_ARG, "prj_dist_thomas: line buffer must lie on a 16-byte boundary");
     OnPlanDevice od(plan->device);
     return cuda_rc(prj::launch_thomas_rows(plan, reinterpret_cast<double2*>(d_lines), kx0, kx1 - kx0,
                                            (cudaStream_t)stream),

@@ -472,7 +472,7 @@ int prj_poisson_fp64_noalloc(int nx, int nz, int ny, double dx, double dz,
  *                     q-major: [q][y - y0][kx - kx_bounds[q]][z].
  *   prj_dist_thomas   Thomas sweeps of the lines kx0 .. kx1-1 held in d_lines as
  *                     [y][kx - kx0][z] over all ny planes (the blocks received
- *                     from all ranks, in rank order).
+ *                     from all ranks, in rank order), on a 16-byte boundary.
  *   prj_dist_unpack   the blocks received back (layout of prj_dist_pack) into the
  *                     planes' spectrum.
  *   prj_dist_inverse  inverse z and x transforms of the planes into d_P_local.

@@ -54,3 +54,16 @@ def test_step_of_misaligned_predictors(cuda_device, oracle, shape, which):
     want = oracle.projection(Uh, Vh, Wh, dx, dz, dt, yu, "consistent", wall)
     for g, w in zip(got, want):
         assert np.abs(g - w).max() <= 1e-12 * np.abs(w).max()
+
+
+def test_rank_lines_off_a_boundary_are_refused(cuda_device):
+    import ctypes
+    import torch
+    import prj
+    import workloads
+    nx, ny, nz = 64, 8, 48
+    _, yu, dx, dz = workloads.poisson_rhs(nx, ny, nz, seed=1)
+    with prj.Plan(nx, nz, ny, dx, dz, prj.bands(yu, "consistent")) as plan:
+        buf = torch.zeros(ny * nz * 4 * 2 + 2, dtype=torch.float64, device="cuda")
+        rc = prj.load_library().prj_dist_thomas(plan.handle, ctypes.c_void_p(buf.data_ptr() + 8), 0, 4, None)
+        assert rc == prj.PRJ_ERR_ARG
