@@ -1,10 +1,13 @@
 """CPU check of the division method of the Thomas forward sweeps (csrc/div_rn.cuh).
 
 The kernels form y = RN(1/D) off the recurrence's chain and then, per quotient,
-q = RN(u y), r = RN(u - D q) (one fused multiply-add, exact here), and return q when
-r == 0, else RN(q + r y) (a second fused multiply-add): Markstein's final correction step.
+q = RN(u y), r = RN(u - D q) (one fused multiply-add, exact here) and RN(q + r y) (a second
+fused multiply-add): Markstein's final correction step, without a branch.  Beside the value the
+function says whether it may differ from RN(u / D): q outside the window [2^-900, 2^1000), but
+for the zero numerators whose sign the step keeps.  The caller then divides plainly.
 Here every rounding is restated with exact rationals (a fused multiply-add is one rounding
-of the exact value; Python rounds int / int and float / float correctly), and the result is
+of the exact value; Python rounds int / int and float / float correctly), the flag with the
+kernel's integer expressions on the words of u, D and q, and the result is
 compared with the correctly rounded quotient u / D bit for bit, signs of zero included.
 The GPU test (test_gpu_division.py) runs the same comparison against __ddiv_rn."""
 import math
@@ -39,24 +42,36 @@ def ieee_div(u: float, D: float) -> float:
     return u / D
 
 
-def div_by_recip(u: float, D: float) -> float:
-    """The kernels' division for a pivot 2^-40 <= |D| <= 2^1000: the correction step when
-    2^-900 <= |q| < 2^1000 (or u = 0), else IEEE division."""
-    assert 2.0 ** -40 <= abs(D) <= 2.0 ** 1000
-    y = 1.0 / D  # RN(1/D), as __drcp_rn
-    q = u * y  # RN(u y)
-    if u != 0.0 and not (2.0 ** -900 <= abs(q) < 2.0 ** 1000):
-        return ieee_div(u, D)
-    r = fma(-D, q, u)
-    return q if r == 0.0 else fma(r, y, q)
+def words(x: float):
+    """The high and low 32-bit words of a double."""
+    w = struct.unpack("<Q", struct.pack("<d", x))[0]
+    return w >> 32, w & 0xFFFFFFFF
 
 
 def correction_step(u: float, D: float) -> float:
-    """The correction step alone (no window), to show where it stops being exact."""
-    y = 1.0 / D
-    q = u * y
+    """RN(q + r y): the value that the kernels' function returns for every u and D."""
+    y = 1.0 / D  # RN(1/D), as __drcp_rn
+    q = u * y  # RN(u y)
+    if math.isinf(q) or math.isnan(q):
+        return math.nan  # outside the window: the value is not used
     r = fma(-D, q, u)
-    return q if r == 0.0 else fma(r, y, q)
+    return fma(r, y, q)
+
+
+def outside(u: float, D: float) -> bool:
+    """The flag that the kernels' function sets: the value above may differ from RN(u / D)."""
+    hq = words(u * (1.0 / D))[0] & 0x7FFFFFFF
+    q_in = (hq - 0x07B00000) & 0xFFFFFFFF < 0x7E700000 - 0x07B00000
+    (hu, lu), hd = words(u), words(D)[0]
+    not_zero = (hu & ~(hd & 0x80000000) & 0xFFFFFFFF) | lu
+    return not q_in and not_zero != 0
+
+
+def div_by_recip(u: float, D: float) -> float:
+    """The kernels' division for a pivot 2^-40 <= |D| <= 2^1000: the step, redone by IEEE division
+    where the flag is set."""
+    assert 2.0 ** -40 <= abs(D) <= 2.0 ** 1000
+    return ieee_div(u, D) if outside(u, D) else correction_step(u, D)
 
 
 def bits(x: float) -> int:
@@ -90,20 +105,28 @@ def test_zero_numerator_keeps_the_quotient_sign(u, D):
     assert bits(div_by_recip(u, D)) == bits(u / D)
 
 
-def test_exact_quotients_take_the_product():
-    # r == 0 exactly: q is u / D already
+def test_exact_quotients_come_back_from_the_step():
+    # r == 0 exactly: q is u / D already, and adding 0 y leaves it
     for u, D in ((6.0, 3.0), (-1.5, 0.5), (1.0, 1024.0), (7.0, -7.0)):
-        assert div_by_recip(u, D) == u / D
+        assert not outside(u, D)
+        assert bits(correction_step(u, D)) == bits(u / D)
 
 
-def test_select_is_what_keeps_minus_zero():
-    # without the r == 0 select, fma(+0, y, -0) = +0 would replace -0 / D = -0 for D > 0
-    u, D = -0.0, 3.0
-    y = 1.0 / D
-    q = u * y
-    r = fma(-D, q, u)
-    assert r == 0.0 and bits(fma(r, y, q)) != bits(u / D)
-    assert bits(div_by_recip(u, D)) == bits(u / D)
+def test_which_zeros_the_step_keeps():
+    """Only -0 / D with D > 0 comes out wrong (+0 y + -0 = +0), and only that one is flagged."""
+    for u in (0.0, -0.0):
+        for D in (3.0, -3.0, 2.0 ** -40, -(2.0 ** 1000)):
+            wrong = bits(correction_step(u, D)) != bits(u / D)
+            assert wrong == outside(u, D) == (math.copysign(1.0, u) < 0 < D), (u, D)
+
+
+def test_which_quotients_are_flagged():
+    """The window's bounds, subnormals and infinities; a non-zero u whose low word is zero."""
+    for D in (1.0, -1.0):
+        assert not outside(2.0 ** -900, D) and outside(math.nextafter(2.0 ** -900, 0.0), D)
+        assert not outside(math.nextafter(2.0 ** 1000, 0.0), D) and outside(2.0 ** 1000, D)
+        for u in (5e-324, -5e-324, 2.0 ** -1022, -(2.0 ** -1000), math.inf, -math.inf, math.nan):
+            assert outside(u, D), (u, D)
 
 
 @pytest.mark.parametrize("seed", [21, 22])
