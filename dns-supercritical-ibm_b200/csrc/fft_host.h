@@ -41,7 +41,7 @@ inline int pass_orders(int n) {
 
 // Fewest passes over the radices 2 .. 11 and 13 (each pass is a round trip through shared
 // memory and a barrier), among those the smallest largest radix (registers), found by trying
-// every multiset in descending order; 0 if n has a larger prime factor.
+// every multiset in descending order; -1 if n has a larger prime factor or needs more passes.
 inline int short_radices(int n, int most, int left, int* fac) {
     if (n == 1) return 0;
     if (left == 0) return -1;

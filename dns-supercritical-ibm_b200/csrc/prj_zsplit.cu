@@ -77,18 +77,18 @@ struct ZanyArgs {
     int nrow_total, nz, rb;
     FftDev f;
     const double2* tw;
-    void* X;
+    double2* X;
 };
-template <int DIR, typename T>
+template <int DIR>
 __global__ void __launch_bounds__(256, PRJ_FFT_MINB) k_zfft_any(const ZanyArgs a) {
     extern __shared__ __align__(16) double2 zs[];
     const size_t row0 = (size_t)blockIdx.x * a.rb;
     const int nr = (int)min((size_t)a.rb, (size_t)a.nrow_total - row0), tot = nr * a.nz;
-    T* X = static_cast<T*>(a.X) + row0 * a.nz;
-    for (int i = threadIdx.x; i < tot; i += blockDim.x) zs[i] = to_d2(X[i]);
+    double2* X = a.X + row0 * a.nz;
+    for (int i = threadIdx.x; i < tot; i += blockDim.x) zs[i] = X[i];
     __syncthreads();
     const double2* r = fft_rows<DIR>(zs, zs + (size_t)a.rb * a.nz, nr, a.nz, a.f, a.tw);
-    for (int i = threadIdx.x; i < tot; i += blockDim.x) from_d2(X[i], r[i]);
+    for (int i = threadIdx.x; i < tot; i += blockDim.x) X[i] = r[i];
 }
 
 // k_zfft_pass: one CTA per group of rb rows (zsplit_tiles.cuh)
@@ -201,8 +201,7 @@ cudaError_t launch_zfft_pass(const prj_plan* pl, int dir, void* X, int rows_per_
 }
 
 // the same for lengths with a prime factor above 13: natural order in and out
-template <typename T>
-cudaError_t launch_zfft_any(const prj_plan* pl, int dir, void* X, int rows_per_plane, cudaStream_t st) {
+cudaError_t launch_zfft_any(const prj_plan* pl, int dir, double2* X, int rows_per_plane, cudaStream_t st) {
     const Geometry& g = pl->g;
     ZanyArgs a{};
     a.nrow_total = g.ny * rows_per_plane;
@@ -215,7 +214,7 @@ cudaError_t launch_zfft_any(const prj_plan* pl, int dir, void* X, int rows_per_p
     while (a.rb > 1 && (size_t)2 * a.rb * g.nz * sizeof(double2) > (size_t)48 * 1024) a.rb /= 2;
     const size_t smem = (size_t)2 * a.rb * g.nz * sizeof(double2);
     const unsigned grid = (unsigned)((a.nrow_total + a.rb - 1) / a.rb);
-    auto kernel = dir < 0 ? k_zfft_any<-1, T> : k_zfft_any<+1, T>;
+    auto kernel = dir < 0 ? k_zfft_any<-1> : k_zfft_any<+1>;
     cudaError_t e = allow_smem(kernel, smem);
     if (e != cudaSuccess) return e;
     kernel<<<grid, 256, smem, st>>>(a);
@@ -223,11 +222,12 @@ cudaError_t launch_zfft_any(const prj_plan* pl, int dir, void* X, int rows_per_p
 }
 
 // in-place z FFT of every spectral row of one buffer: dir < 0 forward (natural ->
-// slot order), dir > 0 inverse (slot order -> natural); needs pl->zd.ok.
+// slot order), dir > 0 inverse (slot order -> natural).
 // `rows_per_plane` rows of T storage per y plane.
 template <typename T>
 cudaError_t launch_zfft_t(const prj_plan* pl, int dir, void* X, int rows_per_plane, cudaStream_t st) {
-    if (!pl->zd.ok) return launch_zfft_any<T>(pl, dir, X, rows_per_plane, st);
+    if constexpr (sizeof(T) == sizeof(double2))  // the mixed path refuses other lengths
+        if (!pl->zd.ok) return launch_zfft_any(pl, dir, static_cast<double2*>(X), rows_per_plane, st);
     {
         const cudaError_t e = launch_zfft_pass<T>(pl, dir, X, rows_per_plane, st);
         if (e != cudaErrorNotSupported) return e;
