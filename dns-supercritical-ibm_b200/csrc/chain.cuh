@@ -48,14 +48,19 @@ inline cudaError_t launch_chained(bool chained, void (*kernel)(P...), dim3 grid,
     return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
-// Clusters of C CTAs along x that the device holds at once (a cluster's CTAs share one GPC, so
-// this is less than the free CTA slots divided by C: 15 clusters of 8 at one CTA per SM of 148).
-// 0 when the query fails.  Kernels asked about here are launched with the limit set here, the
+// Are `count` clusters of C CTAs along x resident at once, of a kernel of which `slots` CTAs are?
+// A cluster's CTAs share one GPC, so fewer are than slots / C (15 clusters of 8 at one CTA per SM
+// of 148), and the runtime is asked, which takes some 40 us; but not for what the slots cannot
+// hold, for single CTAs, or for clusters on half of the slots, which always fit: a GPC of g >= C
+// slots uses C floor(g / C) >= g / 2 of them.  Kernels asked about here are launched with the limit set here, the
 // device's: one value for all callers, so a thread that creates a plan takes nothing from one
 // that launches.
 constexpr int kSmemLimit = 227 * 1024;
 template <typename K>
-inline int resident_clusters(K kernel, unsigned threads, size_t smem, unsigned C) {
+inline bool clusters_resident(K kernel, unsigned threads, size_t smem, unsigned C, int count, int slots) {
+    const long long need = (long long)count * C;
+    if (need > slots) return false;
+    if (C == 1 || 2 * need <= slots) return true;
     int most = 0;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(C);
@@ -70,9 +75,9 @@ inline int resident_clusters(K kernel, unsigned threads, size_t smem, unsigned C
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit) != cudaSuccess ||
         cudaOccupancyMaxActiveClusters(&most, kernel, &cfg) != cudaSuccess) {
         cudaGetLastError();
-        return 0;
+        return false;
     }
-    return most;
+    return most >= count;
 }
 
 }  // namespace prj

@@ -162,7 +162,9 @@ void zline_cluster_shape(const prj_plan* pl, int* C_out, int* yb_out) {
         int yb = 8;
         while (yb > 1 && zline_cluster_smem(g.nz, g.mzp, yb, 2) > std::min(most, (size_t)220 * 1024)) yb--;
         if (yb < 2 || yb * C > g.ny) continue;
-        if (resident_clusters(kernel, nt, zline_cluster_smem(g.nz, g.mzp, yb, 2), (unsigned)C) < g.nxh) continue;
+        // per_sm of them fit an SM by their shared memory, and by registers as the kernel is bound
+        if (!clusters_resident(kernel, nt, zline_cluster_smem(g.nz, g.mzp, yb, 2), (unsigned)C, g.nxh, per_sm * pl->sms))
+            continue;
         *C_out = C;
         *yb_out = yb;
         return;

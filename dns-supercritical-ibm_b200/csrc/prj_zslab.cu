@@ -409,11 +409,8 @@ int zslab_planes(const prj_plan* pl) {
         if (C > 8 || H > 256) return false;  // 256 planes: a tensor-map box
         const size_t smem = slab_smem(g.nz, H);
         if (smem + 1024 > (size_t)220 * 1024) return false;
-        // two CTAs per SM by registers.  What cannot fit by SM slots needs no asking, and single
-        // CTAs fill them all; a query takes some 40 us of the plan's creation.
-        const int per_sm = std::min((int)((size_t)228 * 1024 / (smem + 1024)), 2);
-        if ((long long)g.nxh * C > (long long)per_sm * pl->sms) return false;
-        return C == 1 || resident_clusters(kernel, kSlabThreads, smem, (unsigned)C) >= g.nxh;
+        const int per_sm = std::min((int)((size_t)228 * 1024 / (smem + 1024)), 2);  // two by registers
+        return clusters_resident(kernel, kSlabThreads, smem, (unsigned)C, g.nxh, per_sm * pl->sms);
     };
     if (pl->z_planes > 0) {
         // chunks of the kernel that z_mode 1 or 3 runs by default; else planes per CTA here
