@@ -133,7 +133,8 @@ struct prj_plan {
     int zcl_c = 0, zcl_yb = 0;    // CTAs per wavenumber (0: not it; 1: k_zline) and planes per chunk
     bool use_pass = true;         // compile-time pass-plan FFT kernels where the length has one
     int thomas_async = -1;        // Thomas lines streamed through a cp.async shared-memory ring:
-                                  // -1 and 0 never, 1..4 always (ring shape)
+                                  // 0 never, 1..4 always (ring shape), -1 never but for the mixed
+                                  // storage below two CTAs per SM (8 x 2)
     int tz_xp = 1;                // rows per CTA of the pass-plan x kernels
     double* vd_pad = nullptr;     // inv_dy_p_pad (ny+1) of the variable-density step
     double* vd_ih = nullptr;      // 0.5 / rho (halo'd) of the variable-density step (scratch)

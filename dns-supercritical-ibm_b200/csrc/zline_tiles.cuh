@@ -382,7 +382,7 @@ __device__ __forceinline__ void zline_tile(const ZLineArgs& a, const void* tmap,
 }
 
 // arguments of a plan's z solves (FP64 spectrum, pivots, z pass plan; yb from the plan's
-// z_planes tuning or 4; prj_zline.cu)
+// z_planes tuning or 4, the batch kernel's; k_zline and its cluster form set their own)
 ZLineArgs zline_args(const prj_plan* pl);
 
 // shared memory of a tile (alignment slack, mbarriers, row stages, pivot ring, a and a00)

@@ -322,7 +322,8 @@ int prj_batch_destroy(prj_batch* batch);
  *               plan picks by size and the default z_mode is 0, planes per CTA of the on-chip
  *               kernel, if all its CTAs are then resident at once;
  *   z_stages    stages of their copy rings (0 = default, else 2..4; 2..8 for mode 1);
- *   thomas_ring shared-memory ring of the split Thomas kernel: -1 = default (none),
+ *   thomas_ring shared-memory ring of the split Thomas kernel: -1 = default (none, but
+ *               8x2 for the mixed storage where the grid has fewer than two CTAs per SM),
  *               0 = none, 1..4 = shapes 4x4, 8x2, 2x8, 8x3
  *               (planes x stages) for both storages;
  *   mixed_iters refinement passes of PRJ_MODE_FP32_REFINE (default 1, 0..8);

@@ -21,6 +21,7 @@ def test_emulated_ranks_equal_single_gpu(cuda_device, monkeypatch, world, shape)
     bands = prj.bands(yu, "consistent")
     with prj.Plan(nx, nz, ny, dx, dz, bands) as plan:
         plan.set_tuning(z_mode=0)  # the split z kernels, which the ranks run
+        assert plan.launches_per_step() == 6
         ref = to_dev(rhs)
         plan.poisson_fp64(ref)
         ref = from_dev(ref)
@@ -72,6 +73,7 @@ def test_emulated_projection_step_equals_single_gpu(cuda_device, monkeypatch, wo
     wall = (0.01, 0.0, -0.02, 0.03, 0.0, 0.04)
     with prj.Plan.from_yu(nx, nz, dx, dz, yu, "consistent") as plan:
         plan.set_tuning(z_mode=0)  # the split z kernels, which the ranks run
+        assert plan.launches_per_step() == 6
         ref = run_engine(plan, Uh, Vh, Wh, 0.6, wall)
     plans = [prj.Plan.from_yu(nx, nz, dx, dz, yu, "consistent") for _ in range(world)]
     try:

@@ -42,6 +42,7 @@ def test_orders_match_oracle_and_kernel_families_agree(cuda_device, oracle, shap
         for xo in range(nxo):
             for zo in range(nzo):
                 split = _solve(plan, rhs, x_order=xo, z_order=zo, z_mode=0)
+                assert plan.launches_per_step() == 6
                 assert plan.tuning["x_order"] == xo and plan.tuning["z_order"] == zo
                 assert rel_l2(split, Po) <= 1e-12, (xo, zo)
                 line = _solve(plan, rhs, z_mode=3)

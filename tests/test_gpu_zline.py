@@ -26,6 +26,8 @@ def _solve(monkeypatch, zsel, nx, ny, nz, seed, **tuning):
     rhs, yu, dx, dz = workloads.poisson_rhs(nx, ny, nz, seed=seed)
     with prj.Plan(nx, nz, ny, dx, dz, prj.bands(yu, "consistent")) as plan:
         plan.set_tuning(**zsel, **tuning)
+        if zsel is SPLIT:
+            assert plan.launches_per_step() == 6
         t = to_dev(rhs)
         plan.poisson_fp64(t)
         plan.check_error()
@@ -61,6 +63,7 @@ def test_line_kernel_projection_step(cuda_device, monkeypatch):
     for mode, zsel in (("split", SPLIT), ("line", LINE)):
         with prj.Plan.from_yu(nx, nz, dx, dz, yu, "consistent") as plan:
             plan.set_tuning(**zsel)
+            assert plan.launches_per_step() == (6 if zsel is SPLIT else 4)
             out[mode] = run_engine(plan, Uh, Vh, Wh, 0.5)
     for a, b in zip(out["split"][:4], out["line"][:4]):
         np.testing.assert_array_equal(a, b)
@@ -68,8 +71,9 @@ def test_line_kernel_projection_step(cuda_device, monkeypatch):
 
 
 def test_default_rule_and_tuning(cuda_device, monkeypatch):
-    """The per-wavenumber kernel is the default from nx/2+1 >= 2 x the SM count (the split
-    kernels below); the tuning call selects either for any grid with the same results."""
+    """z_mode's default is the per-wavenumber kernel from nx/2+1 >= 2 x the SM count and the split
+    kernels below (where a plan without a tuning picks by size); the tuning call selects either
+    for any grid with the same results."""
     import torch
     import prj
     import workloads
@@ -109,6 +113,7 @@ def test_line_kernel_outside_the_fast_division_window(cuda_device, monkeypatch, 
     for mode, zsel in (("split", SPLIT), ("line", LINE)):
         with prj.Plan(nx, nz, ny, dx, dz, b6) as plan:
             plan.set_tuning(**zsel)
+            assert plan.launches_per_step() == (6 if zsel is SPLIT else 4)
             t = to_dev(rhs)
             plan.poisson_fp64(t)
             out[mode] = from_dev(t)
