@@ -139,12 +139,15 @@ static ZClusterKernel zcluster_kernel(const prj_plan* pl) {
 // kernels): 102 / 118 / 124 at 256 x 128 x 128 (C = 3), 306 / 323 / 366 at 384 x 192 x 192 (C = 2),
 // 212 / 287 / 244 at 96 x 300 x 256 and 79 / 150 / 79 at 48 x 105 x 384 (C = 4; 322 and 96 with 8, the
 // first in two waves), 203 / 426 / 246 at 64 x 300 x 384 (238 with 8).  Lengths above 384 gain
-// little or lose: 82 / 119 / 72 at 64 x 64 x 512, 598 / 1032 / 544 at 96 x 292 x 768.
+// little or lose: 82 / 119 / 72 at 64 x 64 x 512, 598 / 1032 / 544 at 96 x 292 x 768.  So do short chains
+// of the longest rows on one to one and a half CTAs per SM, where some SMs hold two and most one:
+// 72 / - / 65 at 96 x 53 x 384 and 81 / - / 76 at 90 x 53 x 384, but 90 / - / 94 at 96 x 80 x 384, 74 / - /
+// 75 at 128 x 53 x 384 and 54 / - / 57 at 96 x 60 x 256.
 // C = 1 (k_zline) below two wavenumbers per SM, from where z_mode's default takes it: with a
-// wavenumber per SM up to nz = 384 and 1.25 up to 768 (one CTA / three kernels): 517 / 524 at
-// 350 x 100 x 512 and 1054 / 1106 at 400 x 128 x 768, but 933 / 886 at 300 x 200 x 512, 938 / 855 at
-// 300 x 128 x 768, and with four and eight lines per thread 1234 / 1082 at 400 x 100 x 1024, 1061 /
-// 830 at 300 x 60 x 1536.
+// wavenumber per SM up to nz = 384 and 1.25 up to 768, 1.5 for chains below 64 planes (one CTA / three
+// kernels): 412 / 426 at 400 x 72 x 512, 1054 / 1106 at 400 x 128 x 768 and 368 / 394 at 450 x 60 x 512, but
+// 933 / 886 at 300 x 200 x 512, 938 / 855 at 300 x 128 x 768, 184 / 175 at 384 x 36 x 512, and with four
+// and eight lines per thread 1234 / 1082 at 400 x 100 x 1024, 1061 / 830 at 300 x 60 x 1536.
 void zline_cluster_shape(const prj_plan* pl, int* C_out, int* yb_out) {
     *C_out = *yb_out = 0;
     const Geometry& g = pl->g;
@@ -155,6 +158,7 @@ void zline_cluster_shape(const prj_plan* pl, int* C_out, int* yb_out) {
     if (pl->sms <= 0 || !zline_supported(pl)) return;
     const unsigned nt = (unsigned)zl_threads(g.nz, zl_lpt(g.nz));
     const ZClusterKernel kernel = zcluster_kernel(pl);
+    if (kernel && g.nz > 256 && g.ny < 64 && 4 * g.nxh > pl->sms && 8 * g.nxh < 3 * pl->sms) return;
     for (int C = kernel ? 4 : 1; C >= 2; C--) {
         const int per_sm = (g.nxh * C + pl->sms - 1) / pl->sms;
         if (per_sm > zl_minb((int)nt)) continue;
@@ -169,7 +173,8 @@ void zline_cluster_shape(const prj_plan* pl, int* C_out, int* yb_out) {
         *yb_out = yb;
         return;
     }
-    if (g.nz <= 384 ? g.nxh >= pl->sms : g.nz <= 768 && 4 * g.nxh >= 5 * pl->sms) *C_out = 1;
+    const int quarters = g.nz <= 384 ? 4 : g.ny >= 64 ? 5 : 6;  // of a wavenumber per SM, at least
+    if (g.nz <= 768 && 4 * g.nxh >= quarters * pl->sms) *C_out = 1;
 }
 
 cudaError_t launch_zline_cluster(const prj_plan* pl, cudaStream_t st) {

@@ -181,11 +181,12 @@ def test_z_mode_names_the_kernels(cuda_device):
 
 # wavenumbers x CTAs that free SM slots would hold but the GPCs do not, long rows on chip, and
 # k_zline below two wavenumbers per SM at long rows, each slower than the three kernels; clusters of
-# four where more would also be resident
+# four where more would also be resident; short chains of long rows
 @pytest.mark.parametrize("shape,launches", [((32, 68, 768), 6), ((32, 256, 240), 6), ((32, 384, 160), 6),
                                             ((36, 83, 600), 6), ((32, 64, 640), 6), ((300, 24, 1536), 6),
                                             ((300, 100, 1024), 6), ((96, 300, 256), 4), ((48, 105, 384), 4),
-                                            ((32, 400, 384), 4)])
+                                            ((32, 400, 384), 4), ((96, 53, 384), 6), ((384, 36, 512), 6),
+                                            ((384, 66, 512), 4)])
 def test_routes_where_a_second_wave_would_run(cuda_device, shape, launches):
     nx, ny, nz = shape
     got, want, n = _both(nx, ny, nz, _rhs(nx, ny, nz, 6))
