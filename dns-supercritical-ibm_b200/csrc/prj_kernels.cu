@@ -336,10 +336,15 @@ struct CorrArgs {
 // u = u_hat - dt grad P on the whole halo'd box (mod_cfd_subroutines.f90:1124-1152);
 // x/z halos take the periodic image (the halo exchange of :1225-1231), the
 // y slices -1 and ny (and V at k = 0) take the wall values (:1234-1244).
+// CH: launched with launch_chained, its own instance: the two instructions cost every CTA, and
+// there is one per row (37 -> 68 us at 48 x 116 x 512, plainly launched).
+template <bool CH>
 __global__ void __launch_bounds__(128) k_correct(const CorrArgs a) {
     // one block per halo'd x-row (jh, kh): no index division, coalesced along x
-    chain_trigger();
-    chain_wait();
+    if constexpr (CH) {
+        chain_trigger();
+        chain_wait();
+    }
     const int nx = a.nx, nz = a.nz, ny = a.ny;
     const int jh = blockIdx.y;
     const int k = (int)blockIdx.x + a.kh0 - 1;
@@ -527,7 +532,11 @@ cudaError_t launch_correction(const prj_plan* pl, const double* P, const double*
     for (int i = 0; i < 6; i++) a.wall[i] = sc.wall[i];
     if (kh.y1 <= kh.y0) return cudaSuccess;
     const dim3 grid((unsigned)(kh.y1 - kh.y0), (unsigned)(g.nz + 2));
-    return launch_chained(chained(pl), k_correct, grid, 128, 0, st, 1, a);
+    // chained up to 6144 rows, where it hides the launch (us per step, chained / plain: 64.0 / 66.2 at
+    // 200 x 60 x 60, 3844 rows; 41.5 / 42.0 at 128 x 96 x 64 and 38.0 / 37.7 at 64 x 64 x 96, 6468; but
+    // 51.0 / 48.0 at 32 x 100 x 100, 10404, and 99 / 87 at 32 x 100 x 300, 30804)
+    if (chained(pl) && grid.x * grid.y <= 6144u) return launch_chained(true, k_correct<true>, grid, 128, 0, st, 1, a);
+    return launch_chained(false, k_correct<false>, grid, 128, 0, st, 1, a);
 }
 
 cudaError_t launch_stats(const prj_plan* pl, const double* U, const double* V, const double* W, const double* P,

@@ -296,7 +296,7 @@ int bwd_tiles_per_plane(const prj_plan* pl) { return (pl->g.nz + pl->tz_xp - 1) 
 // rows per CTA of the tiled x kernels: a power of two whose padded rows (stride
 // pass_row_stride(m)) fit 32 KB, so that 6 CTAs share an SM; for the plans from m = 768, where
 // that is two rows, 64 KB and 256 threads.  Up to 16 rows for lengths without a plan and
-// m <= 32 (and m <= 64 from 2^15 rows of the grid), 8 for m <= 96 and 4 above: registers hold an SM to six CTAs whatever their size, so
+// m <= 32 (and m <= 64 from 20480 rows of the grid), 8 for m <= 96 and 4 above: registers hold an SM to six CTAs whatever their size, so
 // smaller tiles spread a small grid over more SMs and shorten the last wave, down to 4 rows,
 // whose 64-byte runs of the transposed spectrum still make whole DRAM accesses.  Measured
 // (us per call, 16 / 8 / 4 / 2 rows): Poisson 128x96x64 41.1 / 37.1 / 39.8 / 45.2; step
@@ -305,9 +305,10 @@ int bwd_tiles_per_plane(const prj_plan* pl) { return (pl->g.nz + pl->tz_xp - 1) 
 // 92.4 / 99.8 at 160x80x100.  Where 16 rows still make several waves, their longer runs are worth
 // more: Poisson (16 / 8 / 4 rows) 524 / 544 / 604 at 96x292x768, 202 / 210 / 226 at 96x300x256, 106.5 /
 // 106.7 / 114.4 at 96x100x384, 316 / 327 / 363 at 128x300x384, 157 / 159 / 174 at 128x100x512; 63.3 /
-// 61.8 / 65.8 at 128x128x128; m = 96 keeps 8, 691 / 670 / 715 at 192x300x512.
+// 61.8 / 65.8 at 128x128x128 (16384 rows), forward x of a step 31.2 / 33.2 at 128x45x512 (23040);
+// m = 96 keeps 8, 691 / 670 / 715 at 192x300x512.
 int choose_tz_xp(int m, long long rows) {
-    const bool most = pass_orders(m) == 0 || m <= 32 || (m <= 64 && rows >= 1 << 15);
+    const bool most = pass_orders(m) == 0 || m <= 32 || (m <= 64 && rows >= 20480);
     return std::min(fit_tz_xp(m), most ? 16 : m <= 96 ? 8 : 4);
 }
 
