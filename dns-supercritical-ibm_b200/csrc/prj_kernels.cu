@@ -385,24 +385,42 @@ __global__ void __launch_bounds__(128) k_correct(const CorrArgs a) {
 }
 
 // max |div u| over the interior (mod_get_bulk.f90:94-96) and max |P|
-__global__ void k_stats(int nx, int nz, int ny, double inv_dx, double inv_dz, const double* __restrict__ inv_dy_p,
-                        const double* __restrict__ U, const double* __restrict__ V, const double* __restrict__ W,
-                        const double* __restrict__ P, unsigned long long* out) {
-    // whole x-rows per warp: one index division per row, not two 64-bit ones per point (which
-    // bound the kernel: 47 us at 256 x 128 x 128 for the 134 MB it reads)
+// Whole x-rows per warp: one index division per row, not two 64-bit ones per point (which
+// bound the kernel: 47 us at 256 x 128 x 128 for the 134 MB it reads).  FLAT (rows up to 64
+// points, or below 128 and no multiple of 32; below 2^31 points in all): a point per thread and
+// step, two multiplications by a reciprocal each; whole rows leave lanes and loads in flight idle
+// there.  Step with record less step, us, by rows / by points: 107 / 82 at 48 x 163 x 768, 68 / 58 at 64 x
+// 100 x 512, 125 / 113 at 80 x 163 x 768, 83 / 78 at 100 x 100 x 512; 207 / 219 at 96 x 300 x 768, 252 / 286
+// at 128 x 300 x 768, 66 / 69 at 256 x 128 x 128.
+template <bool FLAT>
+__global__ void k_stats(int nx, int nz, int ny, FastDiv nxdiv, FastDiv nzdiv, double inv_dx, double inv_dz,
+                        const double* __restrict__ inv_dy_p, const double* __restrict__ U, const double* __restrict__ V,
+                        const double* __restrict__ W, const double* __restrict__ P, unsigned long long* out) {
     double dmax = 0.0, pmax = 0.0;
     const size_t hrow = (size_t)nx + 2, hplane = hrow * (size_t)(nz + 2);
-    const int rows = nz * ny, nw = (int)(gridDim.x * blockDim.x) >> 5, lane = threadIdx.x & 31;
-    for (int row = (int)(blockIdx.x * blockDim.x + threadIdx.x) >> 5; row < rows; row += nw) {
-        const int k = row / nz, j = row - k * nz;
-        const size_t h = hidx(nx, nz, 0, j, k);
-        const double *u = U + h, *v = V + h, *w = W + h, *p = P + (size_t)row * nx;
-        const double idy = inv_dy_p[k];
+    const int rows = nz * ny, nthr = (int)(gridDim.x * blockDim.x), lane = threadIdx.x & 31;
+    const int first = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+    auto point = [&](const double* u, const double* v, const double* w, const double* p, double idy) {
+        const double d = (u[1] - u[0]) * inv_dx + (w[hrow] - w[0]) * inv_dz + (v[hplane] - v[0]) * idy;
+        dmax = fmax(dmax, fabs(d));
+        pmax = fmax(pmax, fabs(p[0]));
+    };
+    if constexpr (FLAT) {
+        const long long total = (long long)rows * nx;
+#pragma unroll 2
+        for (long long idx = first; idx < total; idx += nthr) {
+            const int row = fdiv((int)idx, nxdiv), i = (int)idx - row * nx;
+            const int k = fdiv(row, nzdiv), j = row - k * nz;
+            const size_t h = hidx(nx, nz, i, j, k);
+            point(U + h, V + h, W + h, P + idx, inv_dy_p[k]);
+        }
+    } else {
+        for (int row = first >> 5; row < rows; row += nthr >> 5) {
+            const int k = row / nz, j = row - k * nz;
+            const size_t h = hidx(nx, nz, 0, j, k);
+            const double idy = inv_dy_p[k];
 #pragma unroll 4
-        for (int i = lane; i < nx; i += 32) {
-            const double d = (u[i + 1] - u[i]) * inv_dx + (w[i + hrow] - w[i]) * inv_dz + (v[i + hplane] - v[i]) * idy;
-            dmax = fmax(dmax, fabs(d));
-            pmax = fmax(pmax, fabs(p[i]));
+            for (int i = lane; i < nx; i += 32) point(U + h + i, V + h + i, W + h + i, P + (size_t)row * nx + i, idy);
         }
     }
     for (int o = 16; o > 0; o >>= 1) {
@@ -544,10 +562,14 @@ cudaError_t launch_stats(const prj_plan* pl, const double* U, const double* V, c
     const Geometry& g = pl->g;
     cudaError_t e = cudaMemsetAsync(out2, 0, 2 * sizeof(double), st);
     if (e != cudaSuccess) return e;
-    size_t blocks = ((size_t)g.nz * g.ny + 7) / 8;  // a warp per x-row
+    const size_t points = (size_t)g.nx * g.nz * g.ny;
+    const bool flat = (g.nx <= 64 || (g.nx < 128 && g.nx % 32 != 0)) && points < (size_t)1 << 31;
+    size_t blocks = flat ? (points + 255) / 256 : ((size_t)g.nz * g.ny + 7) / 8;  // else a warp per x-row
     const size_t cap = (size_t)sm_count() * 8;
     if (blocks > cap) blocks = cap;
-    k_stats<<<(unsigned)blocks, 256, 0, st>>>(g.nx, g.nz, g.ny, 1.0 / g.dx, 1.0 / g.dz, pl->t.inv_dy_p, U, V, W, P,
+    auto kernel = flat ? k_stats<true> : k_stats<false>;
+    kernel<<<(unsigned)blocks, 256, 0, st>>>(g.nx, g.nz, g.ny, make_fastdiv((unsigned)g.nx), make_fastdiv((unsigned)g.nz),
+                                             1.0 / g.dx, 1.0 / g.dz, pl->t.inv_dy_p, U, V, W, P,
                                              reinterpret_cast<unsigned long long*>(out2));
     return cudaGetLastError();
 }

@@ -163,3 +163,19 @@ def test_basic_z_kernel_matches_oracle(cuda_device, oracle, monkeypatch, shape):
     assert rel_l2(P, Po) <= 1e-12
     for a, b in ((U, Uo), (V, Vo), (W, Wo)):
         assert np.abs(a - b).max() <= 1e-12 * np.abs(b).max()
+
+
+@pytest.mark.parametrize("shape", [(1, 3, 4), (2, 5, 3), (31, 9, 7), (64, 6, 11), (65, 7, 5), (96, 5, 6), (126, 4, 3),
+                                   (128, 3, 5), (300, 7, 2)])
+def test_record_equals_the_fields(cuda_device, oracle, shape):
+    """The step's record by points (short rows) and by whole rows: max|div u| of the fields it
+    returned, to rounding, and max|p| exactly."""
+    import prj
+    import workloads
+    nx, ny, nz = shape
+    Uh, Vh, Wh, yu, dx, dz = workloads.projection_inputs(nx, ny, nz, seed=3)
+    with prj.Plan.from_yu(nx, nz, dx, dz, yu, "reference") as plan:
+        U, V, W, P, st = run_engine(plan, Uh, Vh, Wh, 0.7)
+    idy, _, _ = prj.metrics(yu)
+    assert st["div_maxabs"] == pytest.approx(oracle.div_maxabs(U, V, W, dx, dz, idy), rel=1e-12, abs=1e-13)
+    assert st["p_maxabs"] == np.abs(P).max()
