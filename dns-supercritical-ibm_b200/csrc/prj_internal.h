@@ -220,6 +220,7 @@ inline cudaError_t launch_fwd_x_range(const prj_plan* pl, const double* Uh, cons
 int choose_tz_xd(int m, bool even);
 int choose_tz_xp(int m, long long rows);  // rows per CTA of the tiled x kernels, a grid of `rows` x-rows
 int fit_tz_xp(int m);                    // the most rows per CTA that fit
+int x_tile_rows(const prj_plan* pl);     // rows per CTA of the plan's storage in use
 size_t pass_x_smem(int m, int tz);       // their shared memory
 
 // z direction as separate kernels (prj_zsplit.cu)

@@ -291,7 +291,10 @@ cudaError_t allow_smem(K kernel, size_t bytes) {
 }  // namespace
 
 // CTAs per y plane of the pass-plan inverse x kernel (the width of its partial sums)
-int bwd_tiles_per_plane(const prj_plan* pl) { return (pl->g.nz + pl->tz_xp - 1) / pl->tz_xp; }
+int bwd_tiles_per_plane(const prj_plan* pl) {
+    const int tz = x_tile_rows(pl);
+    return (pl->g.nz + tz - 1) / tz;
+}
 
 // rows per CTA of the tiled x kernels: a power of two whose padded rows (stride
 // pass_row_stride(m)) fit 32 KB, so that 6 CTAs share an SM; for the plans from m = 768, where
@@ -312,7 +315,18 @@ int choose_tz_xp(int m, long long rows) {
     return std::min(fit_tz_xp(m), most ? 16 : m <= 96 ? 8 : 4);
 }
 
-// the most rows that fit (the persistent batch kernel's tiles, whose CTAs take many in a row)
+// The plan's rows per CTA; while its spectrum holds FP32 rows, as many as fit unless its tuning asks
+// for another count than the default: FP32 runs of 4 rows are 32 bytes, and the inverse x transforms
+// of a mixed step took 126 us with 4 rows against 90 with 8 at 256x49x512, 314 / 210 at 256x87x768,
+// 413 / 338 at 384x96x768.
+int x_tile_rows(const prj_plan* pl) {
+    const int m = pl->fx64.m;
+    const bool fp32 = pl->kxs < pl->g.nxh && pl->tz_xp == choose_tz_xp(m, (long long)pl->g.nz * pl->g.ny);
+    return fp32 ? fit_tz_xp(m) : pl->tz_xp;
+}
+
+// the most rows that fit (the persistent batch kernel's tiles, whose CTAs take many in a row, and
+// the mixed storage's)
 int fit_tz_xp(int m) {
     const bool plan = pass_orders(m) > 0;
     int tz = 16;
@@ -373,7 +387,7 @@ cudaError_t launch_bwd_xp_pl(const XArgs& a, const dim3& grid, bool chained, cud
 // x kernels for even nx: the half length's compile-time pass plan, or the runtime radices;
 // cudaErrorNotSupported otherwise (the caller uses k_fwd_xd / k_bwd_xd)
 cudaError_t launch_xpass(const prj_plan* pl, bool fwd, FwdSource src, XArgs a, int ny_launch, cudaStream_t st) {
-    a.tz = pl->tz_xp;
+    a.tz = x_tile_rows(pl);
     if (!pl->use_pass || !a.even || !pl->xd.ok || pass_smem_bytes(a) > (size_t)200 * 1024) return cudaErrorNotSupported;
     const dim3 grid((pl->g.nz + a.tz - 1) / a.tz, ny_launch);
     const bool ch = chained(pl);

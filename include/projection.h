@@ -304,7 +304,8 @@ int prj_batch_destroy(prj_batch* batch);
  * which times candidates and caches the winner per grid size), and the
  * parameters of the mixed path.  Every knob is a plan field: the launchers read
  * nothing else.
- *   x_rows      x-rows per CTA of the x-transform kernels (power of two, 1..16);
+ *   x_rows      x-rows per CTA of the x-transform kernels (power of two, 1..16); at the
+ *               default count the mixed storage and the batch kernel take as many as fit;
  *   z_rows      spectral rows per CTA of the split z-transform kernels (0 = default,
  *               else a power of two, 1..16);
  *   z_mode      0 = z FFT / Thomas / inverse z FFT as three kernels, 1 = one fused
